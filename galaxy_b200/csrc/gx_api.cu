@@ -379,7 +379,7 @@ WalkCfg walk_cfg(const gx_handle* h) {
   c.quad = (h->opt.multipole == GX_MULTIPOLE_QUAD && c.precision == 0) ? 1 : 0;
   c.kahan = (h->opt.flags & GX_FLAG_NO_KAHAN) ? 0 : 1;
   c.stats = (h->opt.flags & GX_FLAG_STATS) ? 1 : 0;
-  c.inside_test = h->theta >= 0.57 ? 1 : 0;
+  c.inside_test = h->theta >= kInsideTheta ? 1 : 0;
   c.block = h->opt.walk_block ? static_cast<int>(h->opt.walk_block) : kWalkThreads;
   c.persistent_ctas = h->opt.walk_ctas_per_sm ? static_cast<int>(h->opt.walk_ctas_per_sm) * h->sm_count : 0;
   gx_tuning t;

@@ -109,7 +109,7 @@ int upload_tables(gx_batch* bt, const std::vector<size_t>& which, bool* inside) 
     // the grouping the system would have alone, so its result equals the alone result
     d.group = system_walk_group(bt->device, bt->opt, s.n);
     in.push_back(d);
-    *inside = *inside || s.theta >= 0.57;
+    *inside = *inside || s.theta >= kInsideTheta;
   }
   make_tables(in, sys, tiles, items);
   // Largest systems' items first, so stealing warps finish together.
@@ -463,7 +463,7 @@ int gx_batch_step(gx_batch* bt, uint64_t steps) {
   for (size_t i = 0; i < all.size(); ++i) all[i] = i;
   bool any_fresh = false;
   for (auto& s : bt->systems) any_fresh = any_fresh || !s.pending;
-  for (auto& s : bt->systems) inside = inside || s.theta >= 0.57;
+  for (auto& s : bt->systems) inside = inside || s.theta >= kInsideTheta;
   cudaEventRecord(bt->e0, bt->stream);
   uint64_t k = 0;
   if (bt->tables_dirty || any_fresh) {

@@ -186,12 +186,12 @@ __device__ __forceinline__ void write_rest(const StepBufs& b, uint32_t gi, const
   pp[3] = make_float4(c.pl.lz, c.pr.lz, c.pl.take, c.pr.take);
   pp[4] = make_float4(c.pl.open, c.pr.open, __uint_as_float(child_code(c.lc, n_total)),
                       __uint_as_float(child_code(c.rc, n_total)));
-  if (theta >= 0.57 || f64rec) {
+  if (theta >= kInsideTheta || f64rec) {
     double ctr[3], hf[3], delta, sz;
     node_geometry(c.cur, ctr, hf, delta, sz);
-    if (theta >= 0.57) {
+    if (theta >= kInsideTheta) {
       // box centre and half extents: read only by the walk's inside test, which binds
-      // only for theta >= 1/sqrt(3) (the walk applies it from 0.57 on)
+      // only from kInsideTheta on
       b.nodeC[gi] = make_float4(__double2float_rn(ctr[0]), __double2float_rn(ctr[1]), __double2float_rn(ctr[2]), 0.f);
       b.nodeD[gi] = make_float4(__double2float_rn(hf[0]), __double2float_rn(hf[1]), __double2float_rn(hf[2]), 0.f);
     }
@@ -575,12 +575,12 @@ __global__ void __launch_bounds__(kBuildLeaves, (QUAD ? 2 : 3) * (256 / kBuildLe
     if (S.kids[i].x == kUnset) continue;
     const uint32_t gi = first + i;
     b.kids[gi] = S.kids[i];
-    if (theta >= 0.57 || f64rec) {
+    if (theta >= kInsideTheta || f64rec) {
       double ctr[3], hf[3], delta, sz;
       node_geometry(S.inr[i], ctr, hf, delta, sz);
-      if (theta >= 0.57) {
+      if (theta >= kInsideTheta) {
         // box centre and half extents: read only by the walk's inside test, which binds
-        // only for theta >= 1/sqrt(3) (the walk applies it from 0.57 on)
+        // only from kInsideTheta on
         b.nodeC[gi] = make_float4(__double2float_rn(ctr[0]), __double2float_rn(ctr[1]), __double2float_rn(ctr[2]), 0.f);
         b.nodeD[gi] = make_float4(__double2float_rn(hf[0]), __double2float_rn(hf[1]), __double2float_rn(hf[2]), 0.f);
       }

@@ -48,7 +48,7 @@ struct StepBufs {
   uint2* kids = nullptr;
   uint32_t* parent = nullptr;
   Agg64* agg64 = nullptr;
-  float4* nodeC = nullptr;   // AABB centre (opening test for theta >= 1/sqrt 3)
+  float4* nodeC = nullptr;   // AABB centre (opening test for theta >= kInsideTheta)
   float4* nodeD = nullptr;   // AABB half extents (same)
   float4* nodeQ = nullptr;   // 2 per node (quadrupole mode)
   double* q64 = nullptr;     // 6 per node (quadrupole mode)
@@ -69,7 +69,7 @@ struct WalkCfg {
   int quad = 0;
   int kahan = 1;
   int stats = 0;
-  int inside_test = 0;  // some system has theta >= 1/sqrt(3)
+  int inside_test = 0;  // some system has theta >= kInsideTheta
   int block = kWalkThreads;
   int persistent_ctas = 0;  // 0 = one warp per item (no stealing)
 };

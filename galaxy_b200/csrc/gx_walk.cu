@@ -244,7 +244,7 @@ namespace {
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
-// Opening test for theta >= 1/sqrt(3): the target inside the child's AABB must open it.
+// Opening test for theta >= kInsideTheta: the target inside the child's AABB must open it.
 // Returns the adjusted (take, open, amb) of a child whose distance test said "take".
 __device__ __forceinline__ void inside_test(const StepBufs& b, const float xh[3], uint32_t gi, bool& take, bool& open,
                                             bool& amb) {
@@ -454,7 +454,7 @@ __device__ __forceinline__ void quad2(float2 dx, float2 dy, float2 dz, float2 in
 // A list holding 32 entries is evaluated by all lanes together (the R lanes of a target
 // take turns over its entries), four entries a lane-iteration with packed FP32: the dense
 // list with no decisions, the undecided list with each target's exact test (FP64
-// re-decision in the band, the inside test for theta >= 1/sqrt 3); the targets that open
+// re-decision in the band, the inside test for theta >= kInsideTheta); the targets that open
 // an undecided entry are recorded in it, and one pass afterwards pushes the opened
 // entries. Rounds, lists and entries are independent of one another, so the walk has no
 // dependent chain of one record per step. While the stack holds more than kWalkDeep
@@ -509,11 +509,11 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
     if (sd.n > 1 && vmask && __ldg(&b.agg64[root].m) > 0.0) {
       const float eps2f = __double2float_rn(dmul(sd.eps, sd.eps));
       const float2 eps2 = f2(eps2f, eps2f);
-      // The inside rule (a target inside a node's box opens it) can only bind for
-      // theta >= 1/sqrt(3); it follows the system's own theta (as the single-system
+      // The inside rule (a target inside a node's box opens it) can only bind from
+      // kInsideTheta; it follows the system's own theta (as the single-system
       // handle's choice of kernel does), so a system's terms and their order do not
       // depend on the other systems of a batch.
-      const bool inside_rule = INSIDE && sd.theta >= 0.57;
+      const bool inside_rule = INSIDE && sd.theta >= kInsideTheta;
       float xh[3] = {0.f, 0.f, 0.f}, xl[3] = {0.f, 0.f, 0.f};
       if (valid) {
         const double4 p = b.leaf64[k];

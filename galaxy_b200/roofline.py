@@ -17,7 +17,7 @@ BUILD = 256            # codes + order (8) and the gathered pos/mass (32) read; 
 #                        kids (8), parent links (8), agg64 (80), pair record (80) and the
 #                        exchange word (8) written (siblings' aggregates are read from
 #                        shared memory below each 256-leaf block, from L2 above it)
-BUILD_INSIDE = 32      # theta >= 1/sqrt(3): box centre and half extents (FP32) per internal node
+BUILD_INSIDE = 32      # theta >= 1.15: box centre and half extents (FP32) per internal node
 BUILD_QUAD = 80        # quadrupole: q64 (48) + FP32 copy (32) per internal node
 WALK = 140             # pair record per internal node (80), target leaf (32) and order (4)
 #                        read, acceleration (24) written; each record read once
@@ -29,7 +29,7 @@ def sort_passes(key64: bool = False, radix_bits: int = 8) -> int:
 
 
 def stage_bytes(n: int, key64: bool = False, quad: bool = False, radix_bits: int = 8, inside: bool = False) -> dict:
-    """Algorithmic bytes of each stage of one step for n particles (inside: theta >= 1/sqrt 3)."""
+    """Algorithmic bytes of each stage of one step for n particles (inside: theta >= 1.15)."""
     kb = 8 if key64 else 4
     passes = sort_passes(key64, radix_bits)
     return {

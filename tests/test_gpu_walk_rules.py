@@ -1,0 +1,37 @@
+"""The FP32 walk's opening decisions where its rules change: around the opening angle from
+which the inside rule can bind (2 / sqrt 3), and at the edges of its target groups, lists
+and batches. Every target takes exactly the oracle's terms, so the counts are equal."""
+
+import os
+
+import numpy as np
+import pytest
+
+import galaxy_b200 as gb
+
+pytestmark = pytest.mark.gpu
+
+THREADS = os.cpu_count() or 1
+
+
+def _check(oracle, pos, mass, theta, eps=0.05, **kw):
+    s = gb.GpuLbvh(1.0, eps, theta, stats=True, **kw)
+    got = s.accelerations(pos, mass=mass)
+    st = s.stats()
+    ref, cnt = oracle.lbvh_accelerations(pos, mass, 1.0, eps, theta, threads=THREADS, stats=True)
+    assert (st["leaf_interactions"], st["far_interactions"]) == (cnt["leaf"], cnt["far"])
+    # FP32 terms and sums: the parity gates of tests/test_gpu_walk.py
+    err = oracle.per_particle_rel_err(got, ref)
+    assert np.median(err) <= 1e-6 and np.percentile(err, 99) <= 1e-5, (np.median(err), err.max())
+
+
+@pytest.mark.parametrize("theta", [0.56, 0.58, 1.0, 1.1499, 1.15, 1.1547, 1.16, 1.5])
+def test_inside_rule(oracle, theta):
+    pos, _, mass = oracle.fixture_cluster(3, 3000)
+    # flat and needle-shaped boxes, coincident particles (zero-size boxes), massless ones
+    pos[:700, 2] = 0.0
+    pos[700:900, 1:] = 0.25
+    pos[900:940] = pos[900]
+    mass[1000:1100] = 0.0
+    for group in (8, 16, 32):
+        _check(oracle, pos, mass, theta, walk_group=group)
