@@ -314,10 +314,24 @@ namespace {
 // 4e-6 band around rcrit^2.
 constexpr float kGroupLo = 1.0f - 0x1p-20f;
 // Per-warp stack and list sizes of the FP32 walk (see WarpLists).
-constexpr int kWalkStack = 512;  // stack entries
-constexpr int kWalkDeep = 224;   // above this many stacked entries a round takes one entry
+constexpr int kWalkStack = 384;  // stack entries
+constexpr int kWalkDeep = kWalkStack - kMaxDepth - 36;  // stack entries the wide rounds may fill
 constexpr int kWalkList = 96;    // entries per list: at most 31 left after an evaluation + 64 a round
 constexpr int kWalkFlush = 32;   // a list is evaluated once it holds this many entries
+// Undecided and near entries together: at most 31 of each are left over and a round adds at
+// most 64; a batch of undecided entries moves at most its own number to the near list.
+constexpr int kWalkPool = 128;
+static_assert(31 + 31 + 64 <= kWalkPool, "undecided and near entries");
+// An entry is evaluated relative to the centre of the targets' box when the box's far
+// corner is at most sqrt(kNearRatio) times as far from it as any target that takes it: the
+// rounding of the two relative coordinates is then a few 2^-24 of their difference. Nearer
+// entries (the warp's own leaves and their neighbours, a few percent) keep float-float
+// coordinates, whose difference is exact to 2^-24 of itself. Measured on the collision of
+// 2^20 (walk, relative error against 64 bits): no near list 4.58 ms 3.4e-8 (a disk of
+// 200,003: 9.2e-8, where 3.9e-8 is reached with one), ratio 1024 4.88 ms 3.25e-8, 256 4.91
+// ms 3.23e-8, 64 4.93 ms 3.22e-8, 16 5.12 ms 3.19e-8, 4 5.56 ms 3.14e-8.
+constexpr float kNearRatio = 256.f;
+constexpr uint32_t kNearCode = 0x40000000u;  // flag of an undecided entry's code (indices are below 2^30)
 constexpr float kGroupHi = 1.0f + 0x1p-20f;
 
 // Order-preserving map of a float onto a signed int (for warp min / max reductions).
@@ -341,20 +355,26 @@ __device__ __forceinline__ void put2(float4* a, int e, float v0, float v1) {
 // Per-warp shared memory of the FP32 walk.
 //   stk: (internal node, target mask) -- the node was opened for the targets in the mask
 //        and its two children are still to be decided for them;
-//   dense list: children every target of their mask takes (leaves, or nodes the group
-//        test accepted for the whole warp): evaluated with no per-target decision, in
-//        FP32 coordinates relative to the centre of the warp's target box;
+//   dense list: children every target of their mask takes, evaluated with no per-target
+//        decision, in FP32 coordinates relative to the centre of the warp's target box;
+//        two entries share each float4: entry e is half (e & 1) of float4 e >> 1;
 //   undecided list: children some targets take and others open (or that need the FP64
-//        re-decision), evaluated with each target's own decision on float-float
-//        coordinates; afterwards each entry holds the mask of the targets that opened it.
-// Two entries share each float4: entry e is half (e & 1) of float4 e >> 1.
+//        re-decision), one field an array: a lane decides one entry for every target;
+//   near list: children to be taken like the dense ones, but so close to the targets,
+//        for the size of the targets' box, that coordinates relative to its centre would
+//        lose bits (kNearRatio): they keep float-float coordinates. It grows down from the
+//        end of the undecided list's arrays;
+//   targets: the float-float coordinates of the warp's targets, negated, two a float4, so
+//        that one broadcast load serves the packed instructions of two targets.
 struct WarpLists {
   uint2 stk[kWalkStack];
   float4 da[kWalkList / 2], db[kWalkList / 2];  // (x, y) (z, m) relative to the box centre
   uint2 dm[kWalkList / 2];                      // target masks
   uint32_t dcode[kWalkList];                    // child codes (quadrupole terms, statistics)
-  float4 ua[kWalkList / 2], ub[kWalkList / 2], uc[kWalkList / 2], ud[kWalkList / 2], ue[kWalkList / 2],
-      uf[kWalkList / 2];  // (xh,yh) (zh,m) (xl,yl) (zl,take) (open,code) (mask,opened)
+  float uxh[kWalkPool], uyh[kWalkPool], uzh[kWalkPool], uxl[kWalkPool], uyl[kWalkPool], uzl[kWalkPool];
+  float um[kWalkPool], utake[kWalkPool], uopen[kWalkPool];
+  uint32_t ucode[kWalkPool], umask[kWalkPool];
+  float4 ta[16], tb[16], tc[16];  // (xh,yh) (zh,xl) (yl,zl) of targets 2i, 2i + 1, negated
   // The targets' padded box as negated faces (lo, hi) and its negated centre o, each
   // duplicated for packed pairs: warp-uniform, read by the rounds only (kept here rather
   // than in 18 registers of every lane).
@@ -363,13 +383,16 @@ struct WarpLists {
 };
 static_assert(sizeof(WarpLists) % 16 == 0, "warp lists keep 16-byte alignment");
 
-// Bound of the stack: a normal round starts at most kWalkDeep entries high and pushes at
-// most one entry per popped one (2 children each, <= 32 popped), an undecided evaluation
-// pushes at most one entry per list entry (< kWalkList), the first deep round at most
-// 2 + 33, and then the depth-first growth adds at most one entry per tree level.
-static_assert(kWalkDeep + 32 + (kWalkList - 1) + 35 + kMaxDepth <= kWalkStack, "walk stack bound");
+// Bound of the stack: a popped entry leads to at most two pushes, at once or from the
+// undecided list, so a round of kk entries raises stacked + undecided entries by at most kk;
+// a round takes no more than keep them within kWalkDeep. At that height it takes one entry
+// and decides its undecided children at once: the stack then grows like a depth-first
+// walk, by at most one entry per tree level. 384 entries: the collisions fill about 250
+// often (320 entries: 20% slower); more only take room from the L1 (512: the walk of a
+// 16,384-particle sphere with quadrupoles 209 us against 190).
+static_assert(kWalkDeep >= 128 && kWalkDeep + kMaxDepth + 4 <= kWalkStack, "walk stack bound");
 
-// Quadrupole mode: each listed internal node's traceless moments, fetched once by the lane
+// Quadrupole mode: each dense internal node's traceless moments, fetched once by the lane
 // that lists it and stored with the two entries of a pair side by side, as the packed
 // evaluation reads them: a = (xx, xx', xy, xy'), b = (xz, xz', yy, yy'), c = (yz, yz', zz, zz').
 // Slots of leaf entries are never written: the evaluation gives them a zero inverse
@@ -377,7 +400,6 @@ static_assert(kWalkDeep + 32 + (kWalkList - 1) + 35 + kMaxDepth <= kWalkStack, "
 // finite values.
 struct WarpQuads {
   float4 dqa[kWalkList / 2], dqb[kWalkList / 2], dqc[kWalkList / 2];
-  float4 uqa[kWalkList / 2], uqb[kWalkList / 2], uqc[kWalkList / 2];
 };
 
 size_t walk_smem_bytes(int block, bool quad) {
@@ -451,16 +473,19 @@ __device__ __forceinline__ void quad2(float2 dx, float2 dy, float2 dz, float2 in
 //   - taken by every target (or a leaf): appended to the dense list;
 //   - opened by every target: pushed back on the stack with the same target mask;
 //   - otherwise: appended to the undecided list.
-// A list holding 32 entries is evaluated by all lanes together (the R lanes of a target
-// take turns over its entries), four entries a lane-iteration with packed FP32: the dense
-// list with no decisions, the undecided list with each target's exact test (FP64
-// re-decision in the band, the inside test for theta >= kInsideTheta); the targets that open
-// an undecided entry are recorded in it, and one pass afterwards pushes the opened
-// entries. Rounds, lists and entries are independent of one another, so the walk has no
-// dependent chain of one record per step. While the stack holds more than kWalkDeep
-// entries, a round takes only the top entry (and evaluates its undecided children at
-// once): the stack then grows like a depth-first walk, by at most one entry per tree
-// level, which bounds it within kWalkStack. Every target takes exactly the reference's
+// An undecided batch of 32 entries is decided one entry a lane, for every target in turn
+// (two at a time, packed FP32 on float-float coordinates read from shared memory; FP64
+// re-decision in the band, the inside test for theta >= kInsideTheta): the masks of the
+// targets that take and that open the entry build up in the lane's registers. (Deciding
+// an entry for a target a lane costs six shared loads, two ballots and a vote an entry;
+// this way none: the collision of 2^20 at theta 0.5, 6.0 -> 4.7 ms, and its error against
+// 64-bit sums 4.1e-8 -> 3.2e-8.) An entry
+// some targets open goes back on the stack for them, one some targets take goes on the
+// dense list for them. The dense list is evaluated a target a lane (the R lanes of a
+// target take turns over its entries), four entries a lane-iteration with packed FP32 and
+// no decisions. Rounds, lists and entries are independent of one another, so the walk has
+// no dependent chain of one record per step. Rounds narrow as the stack fills (kWalkDeep),
+// which bounds it within kWalkStack. Every target takes exactly the reference's
 // set of terms; only the order of summation differs from the FP64 walk. Terms are summed
 // four at a time into a Kahan-compensated accumulator. Node indices are clamped into the
 // record array and the number of records a warp visits is bounded by the system's node
@@ -492,6 +517,7 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
     const int lg = __ffs(G) - 1;
     const uint32_t gmask = G == 32 ? 0xffffffffu : (1u << G) - 1u;
     const int tg = lane & (G - 1), sl = lane >> lg, R = 32 >> lg;
+    const uint32_t tbit = 1u << tg;
     // a target list (active-subset walk) names the item's G targets; else they are the
     // G sorted positions from it.begin
     const uint32_t li = it.begin + tg;
@@ -510,7 +536,7 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
       const float eps2f = __double2float_rn(dmul(sd.eps, sd.eps));
       const float2 eps2 = f2(eps2f, eps2f);
       // The inside rule (a target inside a node's box opens it) can only bind from
-      // kInsideTheta; it follows the system's own theta (as the single-system
+      // kInsideTheta on; it follows the system's own theta (as the single-system
       // handle's choice of kernel does), so a system's terms and their order do not
       // depend on the other systems of a batch.
       const bool inside_rule = INSIDE && sd.theta >= kInsideTheta;
@@ -521,9 +547,17 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
         split_ff(p.y, xh[1], xl[1]);
         split_ff(p.z, xh[2], xl[2]);
       }
-      // negated target coordinates, duplicated for both entries of a packed pair
-      const float2 nxh = f2(-xh[0], -xh[0]), nyh = f2(-xh[1], -xh[1]), nzh = f2(-xh[2], -xh[2]);
-      const float2 nxl = f2(-xl[0], -xl[0]), nyl = f2(-xl[1], -xl[1]), nzl = f2(-xl[2], -xl[2]);
+      if (sl == 0) {
+        float* A = reinterpret_cast<float*>(L.ta + (tg >> 1)) + (tg & 1);
+        float* B = reinterpret_cast<float*>(L.tb + (tg >> 1)) + (tg & 1);
+        float* C = reinterpret_cast<float*>(L.tc + (tg >> 1)) + (tg & 1);
+        A[0] = -xh[0];
+        A[2] = -xh[1];
+        B[0] = -xh[2];
+        B[2] = -xl[0];
+        C[0] = -xl[1];
+        C[2] = -xl[2];
+      }
       // The targets' padded bounding box as negated faces (lo, hi), duplicated, and its
       // centre o (an FP32 value): dense entries and targets are stored relative to o. A
       // target that is not finite turns the box into all of space: no group decisions.
@@ -549,7 +583,7 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
       const uint32_t gmax = n_total - 1;
       const uint32_t max_pairs = sd.n + 64u;
       uint32_t pairs_done = 0;
-      int sp = 1, dl = 0, ul = 0;
+      int sp = 1, dl = 0, ul = 0, nl = 0;  // heights of the stack and the dense, undecided, near lists
       if (lane == 0) L.stk[0] = make_uint2(root, vmask);
       __syncwarp();
       float2 tx = f2(0.f, 0.f), ty = f2(0.f, 0.f), tz = f2(0.f, 0.f);  // per-entry term sums
@@ -580,12 +614,17 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
       };
       auto put_und = [&](int e, float xh_, float yh_, float zh_, float m_, float xl_, float yl_, float zl_,
                          float take, float open, uint32_t code, uint32_t mask) {
-        put2(L.ua, e, xh_, yh_);
-        put2(L.ub, e, zh_, m_);
-        put2(L.uc, e, xl_, yl_);
-        put2(L.ud, e, zl_, take);
-        put2(L.ue, e, open, __uint_as_float(code));
-        put2(L.uf, e, __uint_as_float(mask), 0.f);
+        L.uxh[e] = xh_;
+        L.uyh[e] = yh_;
+        L.uzh[e] = zh_;
+        L.um[e] = m_;
+        L.uxl[e] = xl_;
+        L.uyl[e] = yl_;
+        L.uzl[e] = zl_;
+        L.utake[e] = take;
+        L.uopen[e] = open;
+        L.ucode[e] = code;
+        L.umask[e] = mask;
       };
       // One round: the top kk stack entries, one per lane, each child decided for the
       // whole warp and appended to a list or pushed back.
@@ -637,6 +676,13 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
         const bool opnL = act && !accL && dmax2.x * kGroupHi < r4.x;
         const bool opnR = act && !accR && dmax2.y * kGroupHi < r4.y;
         const bool undL = act && !accL && !opnL, undR = act && !accR && !opnR;
+        // too near for box-relative coordinates: what is taken is farther than dmin, and
+        // than the take threshold
+        const bool nearL = dmax2.x > kNearRatio * fmaxf(dmin2.x, r3.z), nearR = dmax2.y > kNearRatio * fmaxf(dmin2.y, r3.w);
+        const bool nrL = accL && nearL, nrR = accR && nearR;
+        const uint32_t bNL = __ballot_sync(0xffffffffu, nrL), bNR = __ballot_sync(0xffffffffu, nrR);
+        accL = accL && !nearL;
+        accR = accR && !nearR;
         const uint32_t bAL = __ballot_sync(0xffffffffu, accL), bAR = __ballot_sync(0xffffffffu, accR);
         const uint32_t bUL = __ballot_sync(0xffffffffu, undL), bUR = __ballot_sync(0xffffffffu, undR);
         const uint32_t bOL = __ballot_sync(0xffffffffu, opnL), bOR = __ballot_sync(0xffffffffu, opnR);
@@ -644,7 +690,7 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
         const int eUL = ul + __popc(bUL & lt), eUR = ul + __popc(bUL) + __popc(bUR & lt);
         if (QUAD) {
           // the moments of the listed internal children, loaded side by side
-          const bool qL = (accL || undL) && !(cL & kLeafCode), qR = (accR || undR) && !(cR & kLeafCode);
+          const bool qL = accL && !(cL & kLeafCode), qR = accR && !(cR & kLeafCode);
           float4 qaL = make_float4(0.f, 0.f, 0.f, 0.f), qbL = qaL, qaR = qaL, qbR = qaL;
           if (qL) {
             qaL = __ldg(&b.nodeQ[2 * (size_t)cL]);
@@ -654,10 +700,8 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
             qaR = __ldg(&b.nodeQ[2 * (size_t)cR]);
             qbR = __ldg(&b.nodeQ[2 * (size_t)cR + 1]);
           }
-          if (qL && accL) put_quad(Q.dqa, Q.dqb, Q.dqc, eAL, qaL, qbL);
-          if (qL && undL) put_quad(Q.uqa, Q.uqb, Q.uqc, eUL, qaL, qbL);
-          if (qR && accR) put_quad(Q.dqa, Q.dqb, Q.dqc, eAR, qaR, qbR);
-          if (qR && undR) put_quad(Q.uqa, Q.uqb, Q.uqc, eUR, qaR, qbR);
+          if (qL) put_quad(Q.dqa, Q.dqb, Q.dqc, eAL, qaL, qbL);
+          if (qR) put_quad(Q.dqa, Q.dqb, Q.dqc, eAR, qaR, qbR);
         }
         if (accL || accR) {
           // dense entries relative to the box centre: (c_hi - o) + c_lo
@@ -668,9 +712,14 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
           if (accR) put_dense(eAR, rx.y, ry.y, rz.y, r1.w, M, cR);
         }
         dl += __popc(bAL) + __popc(bAR);
-        if (undL) put_und(eUL, chx.x, chy.x, chz.x, r1.z, clx.x, cly.x, clz.x, r3.z, r4.x, cL, M);
-        if (undR) put_und(eUR, chx.y, chy.y, chz.y, r1.w, clx.y, cly.y, clz.y, r3.w, r4.y, cR, M);
+        if (undL || nrL)
+          put_und(undL ? eUL : kWalkPool - 1 - (nl + __popc(bNL & lt)), chx.x, chy.x, chz.x, r1.z, clx.x, cly.x, clz.x,
+                  r3.z, r4.x, cL | (undL && nearL ? kNearCode : 0u), M);
+        if (undR || nrR)
+          put_und(undR ? eUR : kWalkPool - 1 - (nl + __popc(bNL) + __popc(bNR & lt)), chx.y, chy.y, chz.y, r1.w, clx.y,
+                  cly.y, clz.y, r3.w, r4.y, cR | (undR && nearR ? kNearCode : 0u), M);
         ul += __popc(bUL) + __popc(bUR);
+        nl += __popc(bNL) + __popc(bNR);
         const int npush = __popc(bOL) + __popc(bOR);
         if (sp + npush > kWalkStack) {
           bad = true;
@@ -685,15 +734,14 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
         }
         __syncwarp();
       };
-      // The dense terms of pair p (entries 2p, 2p + 1) for this lane's target; on = 0 for
-      // a lane past the list's end (it reads the last pair with no target bit).
-      auto dense_pair = [&](int p, uint32_t on) {
+      // The dense terms of pair p (entries 2p, 2p + 1) for this lane's target.
+      auto dense_pair = [&](int p) {
         const float4 A = L.da[p], B = L.db[p];
         const uint2 Mk = L.dm[p];
         const float2 dx = __fadd2_rn(f2(A.x, A.y), nxr);
         const float2 dy = __fadd2_rn(f2(A.z, A.w), nyr);
         const float2 dz = __fadd2_rn(f2(B.x, B.y), nzr);
-        const bool t0 = (Mk.x >> tg) & on, t1 = (Mk.y >> tg) & on;
+        const bool t0 = (Mk.x & tbit) != 0u, t1 = (Mk.y & tbit) != 0u;
         float i0, i1;
         mono2(dx, dy, dz, f2(B.z, B.w), eps2, t0, t1, tx, ty, tz, i0, i1);
         if (QUAD || STATS) {
@@ -710,119 +758,224 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
         }
       };
       // Evaluate the dense list: every target adds the terms of the entries in its mask.
-      // The R lanes of a target take pairs (2u, 2u + 1) of quads u = q R + sl.
-      auto flush_dense = [&]() {
-        if (dl & 1) {
-          if (lane == 0) put_dense(dl, 0.f, 0.f, 0.f, 0.f, 0u, kLeafCode);
+      // An iteration takes 4 R entries, the R lanes of a target two pairs each; the entries
+      // short of a whole iteration move to the front of the list and wait for more, except
+      // at the walk's end, when empty entries fill the iteration up.
+      const int chunk = 4 * R;
+      auto flush_dense = [&](bool last) {
+        int full = dl & ~(chunk - 1);
+        if (last && full < dl) {
+          full += chunk;
+          if (dl + lane < full) put_dense(dl + lane, 0.f, 0.f, 0.f, 0.f, 0u, kLeafCode);
+          dl = full;
           __syncwarp();
         }
-        const int np = (dl + 1) >> 1;
-        for (int q = 0; 2 * q * R < np; ++q) {
-          const int pa = 2 * (q * R + sl), pb = pa + 1;
-          dense_pair(min(pa, np - 1), pa < np ? 1u : 0u);
-          dense_pair(min(pb, np - 1), pb < np ? 1u : 0u);
+        for (int pa = 2 * sl; 2 * pa < full; pa += 2 * R) {
+          dense_pair(pa);
+          dense_pair(pa + 1);
           fold();
         }
-        dl = 0;
+        const int rest = dl - full;  // < chunk <= 32
+        if (rest && full) {
+          const int e = full + lane;
+          const bool mv = lane < rest;
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+          uint32_t mk = 0, code = 0;
+          float4 qa = v, qb = v;
+          if (mv) {
+            const float* A = reinterpret_cast<const float*>(L.da + (e >> 1)) + (e & 1);
+            const float* B = reinterpret_cast<const float*>(L.db + (e >> 1)) + (e & 1);
+            v = make_float4(A[0], A[2], B[0], B[2]);
+            mk = reinterpret_cast<const uint32_t*>(L.dm + (e >> 1))[e & 1];
+            code = L.dcode[e];
+            if (QUAD) {
+              const float* qA = reinterpret_cast<const float*>(Q.dqa + (e >> 1)) + (e & 1);
+              const float* qB = reinterpret_cast<const float*>(Q.dqb + (e >> 1)) + (e & 1);
+              const float* qC = reinterpret_cast<const float*>(Q.dqc + (e >> 1)) + (e & 1);
+              qa = make_float4(qA[0], qA[2], qB[0], qB[2]);
+              qb = make_float4(qC[0], qC[2], 0.f, 0.f);
+            }
+          }
+          __syncwarp();
+          if (mv) {
+            put_dense(lane, v.x, v.y, v.z, v.w, mk, code);
+            if (QUAD) put_quad(Q.dqa, Q.dqb, Q.dqc, lane, qa, qb);
+          }
+        }
+        dl = rest;
         __syncwarp();  // read before the next round overwrites the list
       };
-      // The undecided pair p for this lane's target; records the targets that open each
-      // entry in the entry (lane sub * G of each sub-lane writes its pair's).
-      auto und_pair = [&](int p, uint32_t on) {
-        const float4 A = L.ua[p], B = L.ub[p], C = L.uc[p], D = L.ud[p], E = L.ue[p], F = L.uf[p];
-        const float2 dx = __fadd2_rn(__fadd2_rn(f2(A.x, A.y), nxh), __fadd2_rn(f2(C.x, C.y), nxl));
-        const float2 dy = __fadd2_rn(__fadd2_rn(f2(A.z, A.w), nyh), __fadd2_rn(f2(C.z, C.w), nyl));
-        const float2 dz = __fadd2_rn(__fadd2_rn(f2(B.x, B.y), nzh), __fadd2_rn(f2(D.x, D.y), nzl));
-        const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-        const uint32_t cL = __float_as_uint(E.z), cR = __float_as_uint(E.w);
-        const bool a0 = (__float_as_uint(F.x) >> tg) & on, a1 = (__float_as_uint(F.y) >> tg) & on;
-        bool tL = a0 && d2.x > D.z, tR = a1 && d2.y > D.w;
-        bool oL = a0 && d2.x < E.x, oR = a1 && d2.y < E.y;
-        bool aL = a0 && !tL && !oL, aR = a1 && !tR && !oR;
-        if (inside_rule) {
-          if (tL && !(cL & kLeafCode)) inside_test(b, xh, cL, tL, oL, aL);
-          if (tR && !(cR & kLeafCode)) inside_test(b, xh, cR, tR, oR, aR);
-        }
-        if (__any_sync(0xffffffffu, aL || aR)) {
-          if (STATS) n_re += (aL ? 1 : 0) + (aR ? 1 : 0);
-          if (aL) resolve(b, k, sd.theta, cL, tL, oL);
-          if (aR) resolve(b, k, sd.theta, cR, tR, oR);
-        }
-        float i0, i1;
-        mono2(dx, dy, dz, f2(B.z, B.w), eps2, tL, tR, tx, ty, tz, i0, i1);
-        if (QUAD) {
-          const float2 iq = f2(tL && !(cL & kLeafCode) ? i0 : 0.f, tR && !(cR & kLeafCode) ? i1 : 0.f);
-          quad2(dx, dy, dz, iq, Q.uqa[p], Q.uqb[p], Q.uqc[p], tx, ty, tz);
-        }
-        if (STATS) {
-          const uint32_t self = kLeafCode | k;
-          n_leaf += (tL && (cL & kLeafCode) && cL != self ? 1 : 0) + (tR && (cR & kLeafCode) && cR != self ? 1 : 0);
-          n_far += (tL && !(cL & kLeafCode) ? 1 : 0) + (tR && !(cR & kLeafCode) ? 1 : 0);
-          n_open += (oL ? 1 : 0) + (oR ? 1 : 0);
-        }
-        const uint32_t m0 = (__ballot_sync(0xffffffffu, oL) >> (sl * G)) & gmask;
-        const uint32_t m1 = (__ballot_sync(0xffffffffu, oR) >> (sl * G)) & gmask;
-        if (tg == 0 && on) reinterpret_cast<uint2*>(L.uf + p)[1] = make_uint2(m0, m1);
-      };
-      // Evaluate the undecided list, then push every entry some target opened.
-      auto flush_und = [&]() {
-        if (ul & 1) {
-          if (lane == 0) put_und(ul, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, kLeafCode, 0u);
+      // Evaluate the near list as flush_dense does the dense one, on float-float coordinates.
+      auto flush_near = [&](bool last) {
+        int full = nl & ~(chunk - 1);
+        if (last && full < nl) {
+          full += chunk;
+          if (nl + lane < full)
+            put_und(kWalkPool - 1 - (nl + lane), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, kLeafCode, 0u);
+          nl = full;
           __syncwarp();
         }
-        const int np = (ul + 1) >> 1;
-        for (int q = 0; 2 * q * R < np; ++q) {
-          const int pa = 2 * (q * R + sl), pb = pa + 1;
-          und_pair(min(pa, np - 1), pa < np ? 1u : 0u);
-          und_pair(min(pb, np - 1), pb < np ? 1u : 0u);
+        const float* TA = reinterpret_cast<const float*>(L.ta + (tg >> 1)) + (tg & 1);
+        const float* TB = reinterpret_cast<const float*>(L.tb + (tg >> 1)) + (tg & 1);
+        const float* TC = reinterpret_cast<const float*>(L.tc + (tg >> 1)) + (tg & 1);
+        const float2 nxh = f2(TA[0], TA[0]), nyh = f2(TA[2], TA[2]), nzh = f2(TB[0], TB[0]);
+        const float2 nxl = f2(TB[2], TB[2]), nyl = f2(TC[0], TC[0]), nzl = f2(TC[2], TC[2]);
+        auto at = [](const float* a, int e) { return *reinterpret_cast<const float2*>(a + e); };
+        for (int q = 2 * sl; 2 * q < full; q += 2 * R) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int e = kWalkPool - 2 - 2 * (q + h);
+            const float2 dx = __fadd2_rn(__fadd2_rn(at(L.uxh, e), nxh), __fadd2_rn(at(L.uxl, e), nxl));
+            const float2 dy = __fadd2_rn(__fadd2_rn(at(L.uyh, e), nyh), __fadd2_rn(at(L.uyl, e), nyl));
+            const float2 dz = __fadd2_rn(__fadd2_rn(at(L.uzh, e), nzh), __fadd2_rn(at(L.uzl, e), nzl));
+            const uint2 Mk = *reinterpret_cast<const uint2*>(L.umask + e);
+            const bool t0 = (Mk.x & tbit) != 0u, t1 = (Mk.y & tbit) != 0u;
+            float i0, i1;
+            mono2(dx, dy, dz, at(L.um, e), eps2, t0, t1, tx, ty, tz, i0, i1);
+            if (QUAD || STATS) {
+              const uint2 cc = *reinterpret_cast<const uint2*>(L.ucode + e);
+              const bool f0 = t0 && !(cc.x & kLeafCode), f1 = t1 && !(cc.y & kLeafCode);
+              if (QUAD && (f0 || f1)) {
+                const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 a0 = f0 ? __ldg(&b.nodeQ[2 * (size_t)cc.x]) : z4, c0 = f0 ? __ldg(&b.nodeQ[2 * (size_t)cc.x + 1]) : z4;
+                const float4 a1 = f1 ? __ldg(&b.nodeQ[2 * (size_t)cc.y]) : z4, c1 = f1 ? __ldg(&b.nodeQ[2 * (size_t)cc.y + 1]) : z4;
+                quad2(dx, dy, dz, f2(f0 ? i0 : 0.f, f1 ? i1 : 0.f), make_float4(a0.x, a1.x, a0.y, a1.y),
+                      make_float4(a0.z, a1.z, a0.w, a1.w), make_float4(c0.x, c1.x, c0.y, c1.y), tx, ty, tz);
+              }
+              if (STATS) {
+                const uint32_t self = kLeafCode | k;
+                n_leaf += (t0 && (cc.x & kLeafCode) && cc.x != self ? 1 : 0) + (t1 && (cc.y & kLeafCode) && cc.y != self ? 1 : 0);
+                n_far += (f0 ? 1 : 0) + (f1 ? 1 : 0);
+              }
+            }
+          }
           fold();
         }
-        __syncwarp();  // the opened masks are written
-        for (int e0 = 0; e0 < ul; e0 += 32) {
-          const int e = e0 + lane;
-          uint32_t om = 0, code = 0;
-          if (e < ul) {
-            om = reinterpret_cast<const uint32_t*>(L.uf + (e >> 1))[2 + (e & 1)];
-            code = reinterpret_cast<const uint32_t*>(L.ue + (e >> 1))[2 + (e & 1)];
-          }
-          const uint32_t bp = __ballot_sync(0xffffffffu, om != 0u);
-          if (sp + __popc(bp) > kWalkStack) {
-            bad = true;
-          } else {
-            if (om) L.stk[sp + __popc(bp & lt)] = make_uint2(code, om);
-            sp += __popc(bp);
+        const int rest = nl - full;  // < chunk <= 32
+        if (rest && full) {
+          const int e = kWalkPool - 1 - (full + min(lane, rest - 1)), d = kWalkPool - 1 - lane;
+          const float v0 = L.uxh[e], v1 = L.uyh[e], v2 = L.uzh[e], v3 = L.um[e], v4 = L.uxl[e], v5 = L.uyl[e], v6 = L.uzl[e];
+          const uint32_t code = L.ucode[e], mk = L.umask[e];
+          __syncwarp();
+          if (lane < rest) put_und(d, v0, v1, v2, v3, v4, v5, v6, 0.f, 0.f, code, mk);
+        }
+        nl = rest;
+        __syncwarp();  // read before it is overwritten
+      };
+      // Decide the last cnt (<= 32) undecided entries, one a lane, for every target: bit t of
+      // tm / om is set when target t takes / opens the entry. The comparisons are sign bits
+      // (take - d2 < 0, d2 - open < 0) shifted into the masks, highest target first; NaN
+      // thresholds become infinite ones, which neither comparison passes.
+      auto und_batch = [&](int cnt) {
+        ul -= cnt;
+        const bool act = lane < cnt;
+        const int e = ul + (act ? lane : 0);
+        const float ex = L.uxh[e], ey = L.uyh[e], ez = L.uzh[e], exl = L.uxl[e], eyl = L.uyl[e], ezl = L.uzl[e];
+        const float em = L.um[e], take = L.utake[e], open = L.uopen[e];
+        const uint32_t fcode = L.ucode[e], code = fcode & ~kNearCode;
+        const uint32_t M = act ? L.umask[e] : 0u;
+        const float2 X = f2(ex, ex), Y = f2(ey, ey), Z = f2(ez, ez), XL = f2(exl, exl), YL = f2(eyl, eyl), ZL = f2(ezl, ezl);
+        const float tk = take == take ? take : INFINITY, no_ = open == open ? -open : INFINITY;
+        const float2 T = f2(tk, tk), N = f2(no_, no_), neg1 = f2(-1.f, -1.f);
+        uint32_t tm = 0, om = 0;
+#pragma unroll 4
+        for (int p = static_cast<int>(G >> 1) - 1; p >= 0; --p) {
+          const float4 A = L.ta[p], B = L.tb[p], C = L.tc[p];
+          const float2 dx = __fadd2_rn(__fadd2_rn(X, f2(A.x, A.y)), __fadd2_rn(XL, f2(B.z, B.w)));
+          const float2 dy = __fadd2_rn(__fadd2_rn(Y, f2(A.z, A.w)), __fadd2_rn(YL, f2(C.x, C.y)));
+          const float2 dz = __fadd2_rn(__fadd2_rn(Z, f2(B.x, B.y)), __fadd2_rn(ZL, f2(C.z, C.w)));
+          const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+          const float2 dt = __ffma2_rn(d2, neg1, T);  // take - d2
+          const float2 dn = __fadd2_rn(d2, N);        // d2 - open
+          tm = __funnelshift_l(__float_as_uint(dt.y), tm, 1);
+          om = __funnelshift_l(__float_as_uint(dn.y), om, 1);
+          tm = __funnelshift_l(__float_as_uint(dt.x), tm, 1);
+          om = __funnelshift_l(__float_as_uint(dn.x), om, 1);
+        }
+        tm &= M;
+        om &= M & ~tm;
+        uint32_t am = M & ~(tm | om);
+        const auto target = [&](int t) { return LIST ? b.targets[it.begin + t] : it.begin + t; };
+        if (inside_rule && !(code & kLeafCode)) {
+          for (uint32_t w = tm; w; w &= w - 1u) {
+            const int t = __ffs(w) - 1;
+            const float* A = reinterpret_cast<const float*>(L.ta + (t >> 1)) + (t & 1);
+            const float xt[3] = {-A[0], -A[2], -reinterpret_cast<const float*>(L.tb + (t >> 1))[t & 1]};
+            bool tk1 = true, op1 = false, am1 = false;
+            inside_test(b, xt, code, tk1, op1, am1);
+            if (!tk1) tm &= ~(1u << t);
+            if (op1) om |= 1u << t;
+            if (am1) am |= 1u << t;
           }
         }
-        ul = 0;
-        __syncwarp();  // pushes visible to the next round; list read before it is refilled
+        if (__any_sync(0xffffffffu, am != 0u)) {
+          if (STATS) n_re += __popc(am);
+          for (uint32_t w = am; w; w &= w - 1u) {
+            const int t = __ffs(w) - 1;
+            bool tk1, op1;
+            resolve(b, target(t), sd.theta, code, tk1, op1);
+            if (tk1) tm |= 1u << t;
+            if (op1) om |= 1u << t;
+          }
+          __syncwarp();
+        }
+        const bool nr = tm != 0u && (fcode & kNearCode), dn = tm != 0u && !nr;
+        const uint32_t bo = __ballot_sync(0xffffffffu, om != 0u);
+        const uint32_t bt = __ballot_sync(0xffffffffu, dn), bn = __ballot_sync(0xffffffffu, nr);
+        if (sp + __popc(bo) > kWalkStack) {
+          bad = true;
+        } else {
+          if (om) L.stk[sp + __popc(bo & lt)] = make_uint2(code, om);
+          sp += __popc(bo);
+        }
+        __syncwarp();  // every lane has read its entry before a near one may take a slot of the batch
+        if (nr) put_und(kWalkPool - 1 - (nl + __popc(bn & lt)), ex, ey, ez, em, exl, eyl, ezl, 0.f, 0.f, code, tm);
+        nl += __popc(bn);
+        if (dn) {
+          const int d = dl + __popc(bt & lt);
+          put_dense(d, (ex + L.no[0].x) + exl, (ey + L.no[1].x) + eyl, (ez + L.no[2].x) + ezl, em, tm, code);
+          if (QUAD && !(code & kLeafCode))
+            put_quad(Q.dqa, Q.dqb, Q.dqc, d, __ldg(&b.nodeQ[2 * (size_t)code]), __ldg(&b.nodeQ[2 * (size_t)code + 1]));
+        }
+        dl += __popc(bt);
+        if (STATS) n_open += __popc(om);
+        __syncwarp();  // pushes and entries visible; the batch read before it is overwritten
       };
       for (;;) {
         if (__any_sync(0xffffffffu, bad)) break;
+        if (dl >= kWalkFlush) flush_dense(false);
+        if (nl >= kWalkFlush) flush_near(false);
         if (sp == 0) {
           if (ul == 0) break;
-          flush_und();
+          und_batch(min(32, ul));
           continue;
         }
-        const bool deep = sp > kWalkDeep;
-        const int kk = deep ? 1 : min(32, sp);
+        const int kk = max(1, min(min(32, sp), kWalkDeep - sp - ul));
+        const bool deep = kk == 1;
         pairs_done += kk;
         if (pairs_done > max_pairs) {
           bad = true;
           break;
         }
         round(kk);
-        if (dl >= kWalkFlush) flush_dense();
-        if (ul >= kWalkFlush || (deep && ul > 0)) flush_und();
+        while (ul >= kWalkFlush || (deep && ul > 0)) {
+          if (dl >= kWalkFlush) flush_dense(false);
+          if (nl >= kWalkFlush) flush_near(false);
+          und_batch(min(32, ul));
+        }
       }
-      if (dl > 0 && !__any_sync(0xffffffffu, bad)) flush_dense();
-      fold();
+      if (!__any_sync(0xffffffffu, bad)) {
+        if (dl > 0) flush_dense(true);
+        if (nl > 0) flush_near(true);
+      }
       __syncwarp();  // the next item's stack writes must not race this item's last reads
     }
     if (__any_sync(0xffffffffu, bad) && lane == 0) raise_err(b.ctl, kErrBadIndex);
-    float ax = KAHAN ? __fsub_rn(sxy.x, cxy.x) : sxy.x;
-    float ay = KAHAN ? __fsub_rn(sxy.y, cxy.y) : sxy.y;
-    float az = KAHAN ? __fsub_rn(sz, cz) : sz;
-    // the R lanes of a target hold partial sums over disjoint entries
+    // The sums leave FP32 here: the compensation is applied, and the R lanes of a target
+    // (partial sums over disjoint entries) are added, in FP64.
+    double ax = KAHAN ? static_cast<double>(sxy.x) - cxy.x : sxy.x;
+    double ay = KAHAN ? static_cast<double>(sxy.y) - cxy.y : sxy.y;
+    double az = KAHAN ? static_cast<double>(sz) - cz : sz;
     for (int o = G; o < 32; o <<= 1) {
       ax += __shfl_xor_sync(0xffffffffu, ax, o);
       ay += __shfl_xor_sync(0xffffffffu, ay, o);
@@ -830,9 +983,9 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
     }
     if (valid && sl == 0) {
       const uint32_t o = b.order[k];
-      b.acc[3 * (size_t)o + 0] = dmul(static_cast<double>(ax), sd.g);
-      b.acc[3 * (size_t)o + 1] = dmul(static_cast<double>(ay), sd.g);
-      b.acc[3 * (size_t)o + 2] = dmul(static_cast<double>(az), sd.g);
+      b.acc[3 * (size_t)o + 0] = dmul(ax, sd.g);
+      b.acc[3 * (size_t)o + 1] = dmul(ay, sd.g);
+      b.acc[3 * (size_t)o + 2] = dmul(az, sd.g);
     }
     if (STATS) {
       n_leaf = warp_sum64(n_leaf);

@@ -35,3 +35,22 @@ def test_inside_rule(oracle, theta):
     mass[1000:1100] = 0.0
     for group in (8, 16, 32):
         _check(oracle, pos, mass, theta, walk_group=group)
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 9, 31, 32, 33, 63, 65, 129, 1025])
+@pytest.mark.parametrize("theta", [0.0, 0.3, 0.8])
+def test_list_edges(oracle, n, theta):
+    pos, _, mass = oracle.fixture_cluster(n, n)
+    mass[: n // 4] = 0.0  # NaN thresholds: decided in FP64
+    for group in (8, 16, 32):
+        _check(oracle, pos, mass, theta, walk_group=group)
+
+
+@pytest.mark.parametrize("n", [33, 1025])
+def test_list_edges_quad(oracle, n):
+    pos, _, mass = oracle.fixture_cluster(n, n)
+    ref = oracle.lbvh_accelerations_quad(pos, mass, 1.0, 0.05, 0.6, threads=THREADS)
+    for group in (8, 16, 32):
+        got = gb.GpuLbvh(1.0, 0.05, 0.6, multipole="quad", walk_group=group).accelerations(pos, mass=mass)
+        err = oracle.per_particle_rel_err(got, ref)
+        assert np.median(err) <= 1e-6 and np.percentile(err, 99) <= 1e-5
