@@ -112,7 +112,7 @@ size_t Arena::bytes_for(size_t n, size_t nsys, int quad, int f64rec) {
   s += 2 * n * 16;                            // nodeC, nodeD
   s += n * 8;                                 // slots
   if (quad) s += 2 * n * 16 + 6 * n * 8;
-  if (f64rec) s += n * sizeof(Node64);
+  if (f64rec) s += n * (sizeof(Rec64) + 4);
   s += tiles * sizeof(TileDesc) + (n / 8 + nsys + 1) * sizeof(WalkItem);
   s += nsys * (sizeof(SysDesc) + sizeof(Bounds) + 48 + kHistWords * 4);
   s += tiles * kStatusWordsPerTile * 4 + 64;
@@ -166,7 +166,10 @@ cudaError_t Arena::ensure(size_t n, size_t tiles, size_t items, size_t nsys, int
     GX_A(b.nodeQ, 2 * nn, float4);
     GX_A(b.q64, 6 * nn, double);
   }
-  if (f) GX_A(b.node64, nn, Node64);
+  if (f) {
+    GX_A(b.rec64, nn, Rec64);
+    GX_A(b.leaf_next, nn, uint32_t);
+  }
   GX_A(b.slots, nn, unsigned long long);
   TileDesc* tl = nullptr;
   GX_A(tl, nt, TileDesc);
@@ -457,8 +460,7 @@ void enqueue_tree(gx_handle* h, const StepBufs& b, int kick, int pending, bool t
   if (timed) cudaEventRecord(h->ev[2], st);
   {
     NvtxRange r("gx.build");
-    launch_build(b, h->opt.multipole == GX_MULTIPOLE_QUAD && h->opt.precision != GX_PREC_F64,
-                 h->opt.precision == GX_PREC_F64, st);
+    launch_build(b, h->opt.multipole == GX_MULTIPOLE_QUAD && h->opt.precision != GX_PREC_F64, st);
   }
   if (timed) cudaEventRecord(h->ev[3], st);
 }
@@ -749,7 +751,8 @@ int walk_active(gx_handle* h, size_t n, size_t n_active, const uint32_t* active,
   // 4 lanes 3.3 / 3.0 / 3.6 / 6.9 / 16.0, 8 lanes 4.2 / 3.2 / 3.2 / 5.1 / 9.8, 32 lanes
   // 8.0 / 5.4 / 3.8 / 3.8 / 5.3; the full walk takes 9.5).
   const double frac = static_cast<double>(n_active) / static_cast<double>(n);
-  const uint32_t group = frac >= 0.08 ? 32u : frac >= 0.04 ? 16u : frac >= 0.015 ? 8u : 4u;
+  // The FP64 walk's lanes walk by themselves, so it always fills its warps.
+  const uint32_t group = h->opt.precision == GX_PREC_F64 || frac >= 0.08 ? 32u : frac >= 0.04 ? 16u : frac >= 0.015 ? 8u : 4u;
   launch_active_targets(b, a.active, na, group, a.inv, a.flags, a.chunks, a.list, count, a.items, h->stream);
   StepBufs bl = b;  // the same tree, walked for the listed targets only
   bl.targets = a.list;
@@ -1401,7 +1404,7 @@ int gx_stage_build(gx_handle* h, size_t n, const uint32_t* sorted_codes, const d
   GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, sorted_mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   const int quad = h->opt.multipole == GX_MULTIPOLE_QUAD && h->opt.precision != GX_PREC_F64;
   GX_CK(h, cudaMemsetAsync(b.bounds, 0, sizeof(Bounds), h->stream));  // no Morton stage here
-  launch_build(b, quad, h->opt.precision == GX_PREC_F64, h->stream);
+  launch_build(b, quad, h->stream);
   std::vector<uint2> kids(n > 1 ? n - 1 : 1);
   std::vector<Agg64> agg(n > 1 ? n - 1 : 1);
   std::vector<double4> leaf(n);

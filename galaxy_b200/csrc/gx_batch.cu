@@ -143,7 +143,7 @@ void enqueue_step(gx_batch* bt, int kick, bool inside) {
   launch_morton_hist(b, nullptr, st);
   launch_sort(b, st);
   const int quad = bt->opt.multipole == GX_MULTIPOLE_QUAD && bt->opt.precision != GX_PREC_F64;
-  launch_build(b, quad, bt->opt.precision == GX_PREC_F64, st);
+  launch_build(b, quad, st);
   launch_walk(b, bcfg(bt, inside), st);
 }
 

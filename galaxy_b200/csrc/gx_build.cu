@@ -77,17 +77,17 @@ __device__ __forceinline__ uint32_t child_code(uint32_t u, uint32_t n_total) {
   return u >= n_total ? u - n_total : (kLeafCode | u);
 }
 
-// Geometry of an aggregate as reference_flatten derives it (solvers/src/lbvh.rs:602-613).
-__device__ __forceinline__ void node_geometry(const AggR& a, double ctr[3], double hf[3], double& delta, double& s) {
-  double dv[3];
+// AABB centre and half extents of an aggregate as reference_flatten derives them
+// (solvers/src/lbvh.rs:602-613), rounded to FP32.
+__device__ __forceinline__ void node_box(const AggR& a, float4& ctr, float4& hf) {
+  float c[3], h[3];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    ctr[c] = dmul(dadd(a.mn[c], a.mx[c]), 0.5);
-    hf[c] = dmul(dsub(a.mx[c], a.mn[c]), 0.5);
-    dv[c] = dsub(a.com[c], ctr[c]);
+  for (int k = 0; k < 3; ++k) {
+    c[k] = __double2float_rn(dmul(dadd(a.mn[k], a.mx[k]), 0.5));
+    h[k] = __double2float_rn(dmul(dsub(a.mx[k], a.mn[k]), 0.5));
   }
-  delta = dsqrt(dlen2(dv[0], dv[1], dv[2]));
-  s = dmul(2.0, fmax(hf[0], fmax(hf[1], hf[2])));
+  ctr = make_float4(c[0], c[1], c[2], 0.f);
+  hf = make_float4(h[0], h[1], h[2], 0.f);
 }
 
 // FP32 record of a child: float-float centre of mass, mass, and the d^2 thresholds.
@@ -154,8 +154,8 @@ struct Climb {
 // The records of the internal node just completed, now that its Karras index gi (and so
 // its unified index c.u) is known. write_agg: what a sibling's fold reads (the FP64
 // aggregate and quadrupole); write_rest: what only later stages read (children, parent
-// links of the children, the sibling-pair walk record, the optional box / FP64 /
-// quadrupole walk data).
+// links of the children, the sibling-pair walk record, the optional box / quadrupole
+// walk data).
 template <bool QUAD>
 __device__ __forceinline__ void write_agg(const StepBufs& b, uint32_t gi, const Climb& c) {
   Agg64 a;
@@ -175,7 +175,7 @@ __device__ __forceinline__ void write_agg(const StepBufs& b, uint32_t gi, const 
 
 template <bool QUAD>
 __device__ __forceinline__ void write_rest(const StepBufs& b, uint32_t gi, const Climb& c, uint32_t n_total,
-                                           double theta, int f64rec) {
+                                           double theta) {
   b.kids[gi] = make_uint2(c.lc, c.rc);
   b.parent[c.lc] = c.u;
   b.parent[c.rc] = c.u;
@@ -186,28 +186,13 @@ __device__ __forceinline__ void write_rest(const StepBufs& b, uint32_t gi, const
   pp[3] = make_float4(c.pl.lz, c.pr.lz, c.pl.take, c.pr.take);
   pp[4] = make_float4(c.pl.open, c.pr.open, __uint_as_float(child_code(c.lc, n_total)),
                       __uint_as_float(child_code(c.rc, n_total)));
-  if (theta >= kInsideTheta || f64rec) {
-    double ctr[3], hf[3], delta, sz;
-    node_geometry(c.cur, ctr, hf, delta, sz);
-    if (theta >= kInsideTheta) {
-      // box centre and half extents: read only by the walk's inside test, which binds
-      // only from kInsideTheta on
-      b.nodeC[gi] = make_float4(__double2float_rn(ctr[0]), __double2float_rn(ctr[1]), __double2float_rn(ctr[2]), 0.f);
-      b.nodeD[gi] = make_float4(__double2float_rn(hf[0]), __double2float_rn(hf[1]), __double2float_rn(hf[2]), 0.f);
-    }
-    if (f64rec) {
-      Node64 nd;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        nd.c[k] = ctr[k];
-        nd.h[k] = hf[k];
-        nd.com[k] = c.cur.com[k];
-      }
-      nd.m = c.cur.m;
-      nd.delta = delta;
-      nd.s = sz;
-      b.node64[gi] = nd;
-    }
+  if (theta >= kInsideTheta) {
+    // box centre and half extents: read only by the walk's inside test, which binds
+    // only from kInsideTheta on
+    float4 ctr, hf;
+    node_box(c.cur, ctr, hf);
+    b.nodeC[gi] = ctr;
+    b.nodeD[gi] = hf;
   }
   if (QUAD) {
     b.nodeQ[2 * (size_t)gi] = make_float4(c.q[0], c.q[1], c.q[2], c.q[3]);
@@ -330,7 +315,7 @@ __global__ void __launch_bounds__(kBuildLeaves, (QUAD ? 2 : 3) * (256 / kBuildLe
                                                               const K* __restrict__ codes,
                                                               const uint32_t* __restrict__ order,
                                                               const double* __restrict__ pos,
-                                                              const double* __restrict__ mass, StepBufs b, int f64rec) {
+                                                              const double* __restrict__ mass, StepBufs b) {
   extern __shared__ __align__(16) unsigned char s_build_raw[];
   BuildSmem<QUAD>& S = *reinterpret_cast<BuildSmem<QUAD>*>(s_build_raw);
   // block j covers leaves [L (j % B), L (j % B) + L) of tile j / B (L = kBuildLeaves, B = kTile / L)
@@ -575,28 +560,13 @@ __global__ void __launch_bounds__(kBuildLeaves, (QUAD ? 2 : 3) * (256 / kBuildLe
     if (S.kids[i].x == kUnset) continue;
     const uint32_t gi = first + i;
     b.kids[gi] = S.kids[i];
-    if (theta >= kInsideTheta || f64rec) {
-      double ctr[3], hf[3], delta, sz;
-      node_geometry(S.inr[i], ctr, hf, delta, sz);
-      if (theta >= kInsideTheta) {
-        // box centre and half extents: read only by the walk's inside test, which binds
-        // only from kInsideTheta on
-        b.nodeC[gi] = make_float4(__double2float_rn(ctr[0]), __double2float_rn(ctr[1]), __double2float_rn(ctr[2]), 0.f);
-        b.nodeD[gi] = make_float4(__double2float_rn(hf[0]), __double2float_rn(hf[1]), __double2float_rn(hf[2]), 0.f);
-      }
-      if (f64rec) {
-        Node64 nd;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          nd.c[a] = ctr[a];
-          nd.h[a] = hf[a];
-          nd.com[a] = S.inr[i].com[a];
-        }
-        nd.m = S.inr[i].m;
-        nd.delta = delta;
-        nd.s = sz;
-        b.node64[gi] = nd;
-      }
+    if (theta >= kInsideTheta) {
+      // box centre and half extents: read only by the walk's inside test, which binds
+      // only from kInsideTheta on
+      float4 ctr, hf;
+      node_box(S.inr[i], ctr, hf);
+      b.nodeC[gi] = ctr;
+      b.nodeD[gi] = hf;
     }
   }
   {
@@ -634,7 +604,7 @@ __global__ void __launch_bounds__(kBuildLeaves, (QUAD ? 2 : 3) * (256 / kBuildLe
 template <bool QUAD, typename K>
 __global__ void __launch_bounds__(kTileThreads) k_build_top(const TileDesc* __restrict__ tiles,
                                                             const SysDesc* __restrict__ sys, uint32_t n_total,
-                                                            const K* __restrict__ codes, StepBufs b, int f64rec) {
+                                                            const K* __restrict__ codes, StepBufs b) {
   const uint32_t blk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // pass-1 block of this warp
   if (blk >= b.ntiles * kBuildBlocksPerTile) return;
   const TileDesc t = tiles[blk / kBuildBlocksPerTile];
@@ -698,7 +668,7 @@ __global__ void __launch_bounds__(kTileThreads) k_build_top(const TileDesc* __re
       const uint32_t gamma = is_left ? c.r : c.l - 1;
       const unsigned long long mine = (static_cast<unsigned long long>(c.u) << 32) | (is_left ? c.l : c.r);
       const unsigned long long old = exch_acq_rel(&b.slots[off + gamma], mine);
-      if (level > 0) write_rest<QUAD>(b, gi, c, n_total, theta, f64rec);
+      if (level > 0) write_rest<QUAD>(b, gi, c, n_total, theta);
       if (old == kEmptySlot) break;  // first to arrive: the sibling folds the parent
       const uint32_t sib_u = static_cast<uint32_t>(old >> 32);
       const uint32_t sib_far = static_cast<uint32_t>(old);
@@ -744,7 +714,7 @@ __global__ void __launch_bounds__(kTileThreads) k_build_top(const TileDesc* __re
       c.u = n_total + gi;
       write_agg<QUAD>(b, gi, c);
       if (proot) {
-        write_rest<QUAD>(b, gi, c, n_total, theta, f64rec);
+        write_rest<QUAD>(b, gi, c, n_total, theta);
         b.parent[c.u] = kNoParent;
         break;
       }
@@ -756,13 +726,13 @@ __global__ void __launch_bounds__(kTileThreads) k_build_top(const TileDesc* __re
 namespace {
 
 template <bool QUAD, typename K>
-void launch_build_t(const StepBufs& b, const K* codes, int f64_records, cudaStream_t st) {
+void launch_build_t(const StepBufs& b, const K* codes, cudaStream_t st) {
   const uint32_t blocks1 = b.ntiles * kBuildBlocksPerTile;
   k_build_local<QUAD, K><<<blocks1, kBuildLeaves, sizeof(BuildSmem<QUAD>), st>>>(b.tiles, b.sys, b.n, codes, b.order,
-                                                                                 b.pos, b.mass, b, f64_records);
+                                                                                 b.pos, b.mass, b);
   // one warp per block of pass 1 (its tops: a few each)
   const uint32_t blocks2 = (blocks1 * 32 + kTileThreads - 1) / kTileThreads;
-  k_build_top<QUAD, K><<<blocks2, kTileThreads, 0, st>>>(b.tiles, b.sys, b.n, codes, b, f64_records);
+  k_build_top<QUAD, K><<<blocks2, kTileThreads, 0, st>>>(b.tiles, b.sys, b.n, codes, b);
 }
 
 }  // namespace
@@ -779,21 +749,21 @@ void build_prepare() {
   set(k_build_local<true, uint64_t>, sizeof(BuildSmem<true>));
 }
 
-void launch_build(const StepBufs& b, int quad, int f64_records, cudaStream_t st) {
+void launch_build(const StepBufs& b, int quad, cudaStream_t st) {
   // Every split's global rendezvous slot starts empty (one memset instead of a re-arming
   // atomic per fold, which the next level's release would have to wait for).
   cudaMemsetAsync(b.slots, 0xFF, static_cast<size_t>(b.n) * sizeof(unsigned long long), st);
   const uint64_t* c64 = reinterpret_cast<const uint64_t*>(b.codes);
   if (b.key64) {
     if (quad)
-      launch_build_t<true>(b, c64, f64_records, st);
+      launch_build_t<true>(b, c64, st);
     else
-      launch_build_t<false>(b, c64, f64_records, st);
+      launch_build_t<false>(b, c64, st);
   } else {
     if (quad)
-      launch_build_t<true>(b, static_cast<const uint32_t*>(b.codes), f64_records, st);
+      launch_build_t<true>(b, static_cast<const uint32_t*>(b.codes), st);
     else
-      launch_build_t<false>(b, static_cast<const uint32_t*>(b.codes), f64_records, st);
+      launch_build_t<false>(b, static_cast<const uint32_t*>(b.codes), st);
   }
 }
 

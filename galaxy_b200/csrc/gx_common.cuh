@@ -17,7 +17,8 @@
 //     agg64[i]  = {aabb_min[3], aabb_max[3], com[3], mass} FP64 (bit-exact fold)
 //     nodeC[i], nodeD[i] = AABB centre, half extents (FP32; theta >= kInsideTheta)
 //     nodeQ[i]  = 2 x float4 traceless quadrupole (xx, xy, xz, yy), (yz, zz, 0, 0)
-//     node64[i] = {center[3], half[3], com[3], mass, delta, s}  FP64 walk record
+//     rec64[i]  = {com[3], mass, d^2 thresholds, left child, next}  FP64 walk record, and
+//     leaf_next[k]: the node after leaf k in depth-first order
 #pragma once
 
 #include <cstdint>
@@ -61,14 +62,16 @@ struct Agg64 {
   double m;
 };
 
-struct Node64 {
-  double c[3];
-  double h[3];
+// FP64 walk record of an internal node: its left child (first visited when it is opened)
+// and the node that follows its subtree in depth-first order, as unified indices.
+struct alignas(64) Rec64 {
   double com[3];
   double m;
-  double delta;
-  double s;
+  double lo2, hi2;  // surely opened below lo2, surely taken above hi2 (squared distances)
+  uint32_t left, next;
+  uint32_t pad[2];
 };
+constexpr uint32_t kWalkEnd = 0xFFFFFFFFu;  // next of the last subtree
 
 // Morton bounding cube of one system (solvers/src/lbvh.rs:105-120 convention).
 struct Bounds {

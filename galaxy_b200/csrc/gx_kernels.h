@@ -52,7 +52,8 @@ struct StepBufs {
   float4* nodeD = nullptr;   // AABB half extents (same)
   float4* nodeQ = nullptr;   // 2 per node (quadrupole mode)
   double* q64 = nullptr;     // 6 per node (quadrupole mode)
-  Node64* node64 = nullptr;  // FP64 walk mode
+  Rec64* rec64 = nullptr;           // FP64 walk mode, per internal node
+  uint32_t* leaf_next = nullptr;    // FP64 walk mode, per leaf
   unsigned long long* slots = nullptr;  // climb exchange words, kEmptySlot between builds
   DevCtl* ctl = nullptr;
   // Target list of an active-subset walk (nullptr: every particle is a target). Item i
@@ -88,7 +89,7 @@ void launch_sort_passes(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* v
 // per-system digit histograms of b.codes (when codes come from the host)
 void launch_code_hist(const StepBufs& b, cudaStream_t st);
 // gx_build.cu: gather leaves + bottom-up Karras build and aggregation
-void launch_build(const StepBufs& b, int quad, int f64_records, cudaStream_t st);
+void launch_build(const StepBufs& b, int quad, cudaStream_t st);
 // Per-device set-up of the build kernels (their dynamic shared-memory limit); call with the
 // device current, before any stream capture.
 void build_prepare();
