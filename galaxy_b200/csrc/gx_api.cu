@@ -274,8 +274,10 @@ void tuned_store(int device, const gx_options& opt, int batched, size_t n, const
 
 // Targets a warp of the FP32 walk when nothing is tuned: narrow groups for small systems,
 // whose walk is the latency of few warps (more warps, tighter group boxes), 32 targets
-// for large ones.
-uint32_t default_walk_group(size_t n) { return n < (size_t{1} << 16) ? 8u : n < (size_t{1} << 19) ? 16u : 32u; }
+// for large ones. Measured at 8 / 16 / 32 targets (walk, us): Plummer 16,384 135 / 158 /
+// 217; disk 40,000 162 / 135 / 158; Plummer 100,000 776 / 588 / 580; disk 200,003 1272 /
+// 969 / 926; collisions of 262,144 2435 / 1796 / 1669 and 1,048,576 - / 5423 / 4714.
+uint32_t default_walk_group(size_t n) { return n < (size_t{1} << 15) ? 8u : n < (size_t{1} << 17) ? 16u : 32u; }
 
 uint32_t system_radix_bits(int device, const gx_options& opt, size_t n) {
   if (opt.flags & GX_FLAG_MORTON63) return kRadixBits;
@@ -386,9 +388,13 @@ WalkCfg walk_cfg(const gx_handle* h) {
   c.block = h->opt.walk_block ? static_cast<int>(h->opt.walk_block) : kWalkThreads;
   c.persistent_ctas = h->opt.walk_ctas_per_sm ? static_cast<int>(h->opt.walk_ctas_per_sm) * h->sm_count : 0;
   gx_tuning t;
-  if (!h->opt.walk_block && !h->opt.walk_ctas_per_sm && tuned_lookup(h->device, h->opt, 0, h->n_layout, &t)) {
-    c.block = static_cast<int>(t.walk_block);
-    c.persistent_ctas = static_cast<int>(t.walk_ctas_per_sm) * h->sm_count;
+  if (!h->opt.walk_block && !h->opt.walk_ctas_per_sm) {
+    if (tuned_lookup(h->device, h->opt, 0, h->n_layout, &t)) {
+      c.block = static_cast<int>(t.walk_block);
+      c.persistent_ctas = static_cast<int>(t.walk_ctas_per_sm) * h->sm_count;
+    } else if (c.precision == 0) {
+      c.auto_ctas = (c.quad ? kWalkCtasQuad : kWalkCtas) * h->sm_count;
+    }
   }
   return c;
 }

@@ -65,6 +65,10 @@ struct StepBufs {
   uint32_t group = 32;
 };
 
+// CTAs of kWalkThreads threads per SM that the FP32 walk's shared memory allows, with
+// monopoles and with quadrupoles.
+constexpr int kWalkCtas = 4, kWalkCtasQuad = 3;
+
 struct WalkCfg {
   int precision = 0;  // 0 = FP32, 1 = FP64
   int quad = 0;
@@ -73,6 +77,10 @@ struct WalkCfg {
   int inside_test = 0;  // some system has theta >= kInsideTheta
   int block = kWalkThreads;
   int persistent_ctas = 0;  // 0 = one warp per item (no stealing)
+  // > 0 (with persistent_ctas 0): as many persistent CTAs when there are more items than
+  // their warps. The warps of a block that finish early then take the next items instead
+  // of idling until the block's last one ends (3-5% of the walk from 200,000 particles on).
+  int auto_ctas = 0;
 };
 
 // gx_step.cu

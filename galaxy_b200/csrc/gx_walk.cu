@@ -415,6 +415,10 @@ struct WarpQuads {
   float4 dqa[kWalkList / 2], dqb[kWalkList / 2], dqc[kWalkList / 2];
 };
 
+static_assert(kWalkCtas * ((kWalkThreads / 32) * sizeof(WarpLists) + 1024) <= 227 * 1024 &&
+                  kWalkCtasQuad * ((kWalkThreads / 32) * (sizeof(WarpLists) + sizeof(WarpQuads)) + 1024) <= 227 * 1024,
+              "resident walk blocks");
+
 size_t walk_smem_bytes(int block, bool quad) {
   return static_cast<size_t>(block / 32) * (sizeof(WarpLists) + (quad ? sizeof(WarpQuads) : 0));
 }
@@ -1030,8 +1034,10 @@ template <class K>
 void launch_k(K kern, const StepBufs& b, const WalkCfg& cfg, size_t smem, cudaStream_t st) {
   const int block = cfg.block > 0 ? cfg.block : kWalkThreads;
   const int wpb = block / 32;
-  if (cfg.persistent_ctas > 0) {
-    kern<<<cfg.persistent_ctas, block, smem, st>>>(b, 1);
+  const int ctas = cfg.persistent_ctas > 0 ? cfg.persistent_ctas
+                   : b.nitems > static_cast<uint32_t>(cfg.auto_ctas * wpb) ? cfg.auto_ctas : 0;
+  if (ctas > 0) {
+    kern<<<ctas, block, smem, st>>>(b, 1);
   } else {
     const uint32_t grid = (b.nitems + wpb - 1) / wpb;
     if (grid) kern<<<grid, block, smem, st>>>(b, 0);

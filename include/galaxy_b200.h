@@ -62,7 +62,7 @@ typedef struct gx_options {
   uint32_t walk_block;     /* threads per block of the tree walk: 0 = default (128), else a
                               multiple of 32 up to 128 */
   uint32_t walk_ctas_per_sm; /* >0: persistent work-stealing walk with this many CTAs per SM;
-                                0: tuned default (one warp per item for a single system) */
+                                0: the tuned choice, else by the number of items */
   uint32_t walk_group;     /* targets per warp of the FP32 walk: 8, 16 or 32; 0 = the tuning
                               table's entry for the system's N, else a rule of N. It changes
                               the order in which the walk sums its terms (never which terms),
