@@ -25,9 +25,9 @@
 // coordinates are clamped to the int32 range (monotone, so a clamped query box still
 // covers its ball). One warp serves one target: its lanes walk the query box's buckets
 // 32 at a time as one flattened list. The density warp keeps its candidates (radius,
-// sorted slot) in shared memory and evaluates every bisection step from there (streaming
+// sorted slot) in shared memory and evaluates counts from there (streaming
 // the box again only when more than kCandCap candidates fall inside). It gathers a ball
-// of 2.5 x the bracket seed instead of the reference's 2 x hi = 4 x seed: a comparison
+// of 2.1 to 2.5 x the bracket seed instead of the reference's 2 x hi = 4 x seed: a comparison
 // whose count needs a wider ball is settled by the lower bound of the gathered part when
 // that clears n_ngb, else the gather widens first, so every comparison is the reference's.
 // The hydro warp lists the neighbours that pass a support test, then runs the pair
@@ -51,8 +51,9 @@ constexpr int kSphThreads = 128;                  // one target per warp
 constexpr int kSphWarps = kSphThreads / 32;
 constexpr int kDensThreads = 256;                 // density: one target per warp, 8 a block
 constexpr int kDensWarps = kDensThreads / 32;
-constexpr int kCandCap = 512;                     // density candidates cached per warp
+constexpr int kCandCap = 256;                     // density candidates cached per warp (512 and three blocks an SM: 8% slower)
 constexpr double kLowerBoundMargin = 1.0 + 1e-10; // a partial count this far above n_ngb decides
+constexpr double kSureMargin = 1e-11;             // a count this far from n_ngb settles its side
 constexpr int kPairCap = 128;                     // hydro: neighbour slots listed per warp
 constexpr uint32_t kBoxAxisMax = 1u << 10;        // a query box wider than this scans all
 constexpr uint32_t kBoxCellsMax = 1u << 15;       //   gas instead of its cells
@@ -146,6 +147,21 @@ __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
   return __shfl_sync(kFull, v, 0);
+}
+
+// The sum on every lane (the same bits: each level adds the same two values).
+__device__ __forceinline__ double warp_sum_all(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  return v;
+}
+__device__ __forceinline__ void warp_sum_all2(double& v, double& w) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double a = __shfl_xor_sync(kFull, v, o), b = __shfl_xor_sync(kFull, w, o);
+    v += a;
+    w += b;
+  }
 }
 
 __device__ __forceinline__ double warp_max(double v) {
@@ -323,6 +339,11 @@ __global__ void __launch_bounds__(kFlat) k_sph_seeds(GridDev g, const uint32_t* 
                                                      const uint32_t* __restrict__ mixed,
                                                      const double* __restrict__ cbrt_tab, SphScalars* sc,
                                                      double* __restrict__ seeds) {
+  // The exponents' histogram in shared memory first: nearly all seeds share a few bins, whose
+  // global atomics would run one after another (65,536 gas particles: 50 -> 10 us).
+  __shared__ uint32_t s_hist[2048];
+  for (int i = threadIdx.x; i < 2048; i += kFlat) s_hist[i] = 0u;
+  __syncthreads();
   const double occ = sc->occ_cell, scale = sc->seed_scale, h_cap = sc->h_cap;
   for (uint32_t s = blockIdx.x * kFlat + threadIdx.x; s < g.n; s += gridDim.x * kFlat) {
     const uint32_t b = skey[s];
@@ -341,21 +362,43 @@ __global__ void __launch_bounds__(kFlat) k_sph_seeds(GridDev g, const uint32_t* 
     const double seed = fmin(occ / cb * scale, h_cap);
     seeds[me.w] = seed;
     const uint32_t e = static_cast<uint32_t>(__double_as_longlong(seed) >> 52) & 2047u;
-    atomicAdd(&sc->seed_hist[e], 1u);
+    atomicAdd(&s_hist[e], 1u);
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2048; i += kFlat)
+    if (s_hist[i]) atomicAdd(&sc->seed_hist[i], s_hist[i]);
 }
 
 // The density query cell from the median seed (density.rs:213-217); the cell only sets
 // how a query's work divides into buckets, never which particles it finds.
-__global__ void k_sph_dens_cell(uint32_t n, SphScalars* sc) {
-  uint32_t acc = 0, e = 0;
-  const uint32_t half = n / 2 + 1;
-  for (; e < 2048; ++e) {
-    acc += sc->seed_hist[e];
-    if (acc >= half) break;
+// One block, eight bins a thread.
+__global__ void __launch_bounds__(kFlat) k_sph_dens_cell(uint32_t n, SphScalars* sc) {
+  __shared__ uint32_t s_warp[kFlat / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t v[8], own = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) own += v[i] = sc->seed_hist[8 * threadIdx.x + i];
+  uint32_t incl = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += y;
   }
-  const double med = 1.4142135623730951 * ldexp(1.0, static_cast<int>(min(e, 2046u)) - 1023);  // bin centre
-  sc->dens_cell = fmax(fmin(2.0 * med, 2.0 * sc->h_seed), 1e-12);
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) incl += s_warp[w];
+  const uint32_t half = n / 2 + 1;
+  uint32_t acc = incl - own;
+  if (acc < half && incl >= half) {  // the median's bin is one of this thread's
+    int i = 0;
+    for (; i < 7; ++i) {
+      acc += v[i];
+      if (acc >= half) break;
+    }
+    const uint32_t e = 8 * threadIdx.x + i;
+    const double med = 1.4142135623730951 * ldexp(1.0, static_cast<int>(min(e, 2046u)) - 1023);  // bin centre
+    sc->dens_cell = fmax(fmin(2.0 * med, 2.0 * sc->h_seed), 1e-12);
+  }
 }
 
 __global__ void __launch_bounds__(kFlat) k_sph_hmax(uint32_t n, const double* __restrict__ hs, SphScalars* sc) {
@@ -389,7 +432,7 @@ struct DensArgs {
   const uint32_t* inv;      // gas-local index -> slot of this grid
 };
 
-__global__ void __launch_bounds__(kDensThreads) k_sph_density(DensArgs a) {
+__global__ void __launch_bounds__(kDensThreads, 4) k_sph_density(DensArgs a) {
   __shared__ double s_r[kDensWarps][kCandCap];
   __shared__ uint32_t s_s[kDensWarps][kCandCap];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -402,9 +445,13 @@ __global__ void __launch_bounds__(kDensThreads) k_sph_density(DensArgs a) {
   const uint32_t k = static_cast<uint32_t>(a.g.sc[slot].w);
   const double h_cap = a.sc->h_cap;
   double seed = a.seeds[k];
+  bool warm = false;
   if (a.warm && a.sc->hint_valid) {
     const double hv = a.hs[k];
-    if (isfinite(hv) && hv > 0.0) seed = hv;
+    if (isfinite(hv) && hv > 0.0) {
+      seed = hv;
+      warm = true;
+    }
   }
   double lo = fmin(seed / 2.0, h_cap);
   double hi = fmin(seed * 2.0, h_cap);
@@ -440,10 +487,10 @@ __global__ void __launch_bounds__(kDensThreads) k_sph_density(DensArgs a) {
       __syncwarp();
     }
   };
-  // sum over the candidates of W(r, h), mass-weighted or not
-  // Candidates at r >= 2h add exact zeros (r >= 2h gives r / h >= 2 after rounding) and
-  // are skipped without the division.
-  auto wsum = [&](double h, bool weighted) -> double {
+  // The mass-weighted sum over the candidates of W(r, h), the density. Candidates at r >= 2h
+  // add exact zeros (r >= 2h gives r / h >= 2 after rounding) and are skipped without the
+  // division.
+  auto wsum = [&](double h) -> double {
     double acc = 0.0;
     const double two_h = 2.0 * h, norm = sph_norm(h);
     if (!over) {
@@ -451,7 +498,7 @@ __global__ void __launch_bounds__(kDensThreads) k_sph_density(DensArgs a) {
         const double r = cr[j];
         if (r >= two_h) continue;
         const double t = sph_w_n(r, h, norm);
-        acc += weighted ? a.g.sp[cs[j]].w * t : t;
+        acc += a.g.sp[cs[j]].w * t;
       }
     } else {
       const double R2 = Rc * Rc;
@@ -464,37 +511,139 @@ __global__ void __launch_bounds__(kDensThreads) k_sph_density(DensArgs a) {
           const double r = sqrt(r2);
           if (r < two_h) {
             const double t = sph_w_n(r, h, norm);
-            acc += weighted ? p.w * t : t;
+            acc += p.w * t;
           }
         }
       });
     }
     return warp_sum(acc);
   };
+  // f(r) for the candidates of this lane (r their distance)
+  auto each = [&](auto&& f) {
+    if (!over) {
+      for (uint32_t j = lane; j < ncand; j += 32) f(cr[j]);
+    } else {
+      const double R2 = Rc * Rc;
+      visit_box(a.g, xi.x, xi.y, xi.z, Rc, [&](bool ok, uint32_t s) {
+        if (!ok) return;
+        const double4 p = a.g.sp[s];
+        const double dx = xi.x - p.x, dy = xi.y - p.y, dz = xi.z - p.z;
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        if (r2 <= R2) f(sqrt(r2));
+      });
+    }
+  };
+  // count(h) = (4 pi / 3) (2h)^3 sum W(r, h) = 32 / 3 sum w(r / h), with the kernel's two
+  // pieces as w(q) = max(2 - q, 0)^3 / 4 - max(1 - q, 0)^3.
+  auto shape = [](double q, double& x2, double& x1) {
+    x2 = fmax(2.0 - q, 0.0);
+    x1 = fmax(1.0 - q, 0.0);
+    return fma(0.25 * x2, x2 * x2, -(x1 * x1 * x1));
+  };
   auto count = [&](double h) -> double {
-    const double s = 2.0 * h;
-    return kFourThirdsPi * (s * s * s) * wsum(h, false);
+    double sum = 0.0, x1, x2;
+    const double inv = 1.0 / h;
+    each([&](double r) { sum += shape(r * inv, x2, x1); });
+    return (32.0 / 3.0) * warp_sum_all(sum);
+  };
+  // count(h) and d count / d ln h = 32 / 3 sum q (3/4 x2^2 - 3 x1^2)
+  auto count_slope = [&](double h, double& slope) -> double {
+    double sum = 0.0, ds = 0.0, x1, x2;
+    const double inv = 1.0 / h;
+    each([&](double r) {
+      const double q = r * inv;
+      sum += shape(q, x2, x1);
+      ds = fma(q, fma(0.75 * x2, x2, -3.0 * x1 * x1), ds);
+    });
+    warp_sum_all2(sum, ds);
+    slope = (32.0 / 3.0) * ds;
+    return (32.0 / 3.0) * sum;
+  };
+  auto count_two = [&](double ha, double hb, double& ca, double& cb) {
+    double sa = 0.0, sb = 0.0, x1, x2;
+    const double ia = 1.0 / ha, ib = 1.0 / hb;
+    each([&](double r) {
+      sa += shape(r * ia, x2, x1);
+      sb += shape(r * ib, x2, x1);
+    });
+    warp_sum_all2(sa, sb);
+    ca = (32.0 / 3.0) * sa;
+    cb = (32.0 / 3.0) * sb;
+  };
+  // count grows with h, so one evaluation settles the reference's comparisons on its side of
+  // the root: below (at and under which count < n_ngb) and above (at and over which count >
+  // n_ngb) are evaluated points that clear n_ngb by kSureMargin, far above any rounding.
+  double below = 0.0, above = INFINITY;
+  auto note = [&](double h, double c) {
+    if (c < a.n_ngb * (1.0 - kSureMargin)) below = fmax(below, h);
+    if (c > a.n_ngb * (1.0 + kSureMargin)) above = fmin(above, h);
   };
   // The candidates are every particle within Rc of the target. count(h) needs all within
   // 2h; when 2h > Rc the candidates' sum is a lower bound of it (every term is >= 0),
   // which settles "count >= n_ngb" whenever it clears n_ngb by more than any rounding
   // could move it. Otherwise the gather widens to 2h first: the comparisons are the
-  // reference's, on a gather that is usually a quarter of its 2 * hi ball.
+  // reference's, on a gather that is usually a small part of its 2 * hi ball.
+  auto evaluate = [&](double h) -> double {
+    if (2.0 * h > Rc) {
+      const double part = count(h);
+      if (part >= a.n_ngb * kLowerBoundMargin) {
+        above = fmin(above, h);
+        return part;
+      }
+      gather(2.0 * h);
+    }
+    const double c = count(h);
+    note(h, c);
+    return c;
+  };
   auto less = [&](double h) -> bool {  // count(h) < n_ngb
-    if (2.0 * h <= Rc) return count(h) < a.n_ngb;
-    if (count(h) >= a.n_ngb * kLowerBoundMargin) return false;
-    gather(2.0 * h);
-    return count(h) < a.n_ngb;
+    return h <= below || (h < above && evaluate(h) < a.n_ngb);
   };
   auto greater = [&](double h) -> bool {  // count(h) > n_ngb
-    if (2.0 * h <= Rc) return count(h) > a.n_ngb;
-    if (count(h) >= a.n_ngb * kLowerBoundMargin) return true;
-    gather(2.0 * h);
-    return count(h) > a.n_ngb;
+    return h >= above || (h > below && evaluate(h) > a.n_ngb);
   };
 
   bool bad = false;
-  gather(fmin(2.0 * hi, 2.5 * seed));
+  // The root first: Newton steps in ln h from the seed (steps of the count's h^3 growth while
+  // far away), then certified by the counts a little below and above it. The reference's
+  // bracket, expansion, shrinking and bisection then run over comparisons that those two
+  // points settle, all but one in ten of them without a count. A ball with too many
+  // candidates is shrunk by the same growth before anything is counted in it. (Counting at
+  // each of about 14 points, over the whole box where the seed of a sparse bin was too
+  // large: 65,536 gas particles warm-started in 965 us, cold in 8.5 ms; this way 290 us and
+  // 0.9 ms.)
+  double x = fmin(seed, h_cap);
+  gather(fmin(2.0 * hi, warm ? 2.1 * x : 2.5 * x));
+  for (int step = 0; step < 16 && x > 0.0; ++step) {
+    if (2.0 * x > Rc) gather(2.1 * x);
+    // (a cold seed only, and only at first: beside a dense core the count itself jumps)
+    for (int k = 0; k < 3 && step == 0 && !warm && over && ncand > 2.0 * a.n_ngb; ++k) {
+      x = 0.5 * Rc * cbrt(a.n_ngb / ncand);
+      gather(2.1 * x);
+    }
+    double slope;
+    const double c = count_slope(x, slope);
+    note(x, c);
+    const double f = a.n_ngb / c, d = (a.n_ngb - c) / slope;  // growth left, Newton's step of ln h
+    if (f > 2.0 || f < 0.5) {  // far away (c >= 32 / 3, the target's own term: f < n_ngb)
+      if (c < a.n_ngb && x >= h_cap) break;
+      x = fmin(x * fmin(fmax(cbrt(f), 0.4), 2.0), h_cap);
+      continue;
+    }
+    if (!(fabs(d) < 0.7)) break;
+    const double xn = x * (1.0 + d + 0.5 * d * d);
+    if (fabs(d) < 0.01) {
+      const double w = fmax(2e-5, 2.0 * d * d), ha = xn * (1.0 - w), hb = xn * (1.0 + w);
+      if (2.0 * hb <= Rc) {
+        double ca, cb;
+        count_two(ha, hb, ca, cb);
+        note(ha, ca);
+        note(hb, cb);
+      }
+      if (below > 0.0 && above - below <= 4.0 * w * xn) break;
+    }
+    x = xn;
+  }
   int it = 0;
   while (less(hi) && hi < h_cap) {
     if (++it > kLoopCap) {
@@ -529,7 +678,7 @@ __global__ void __launch_bounds__(kDensThreads) k_sph_density(DensArgs a) {
     h = 0.5 * (lo + hi);
   }
   if (2.0 * h > Rc) gather(2.0 * h);
-  const double rho = wsum(h, true);
+  const double rho = wsum(h);
   if (lane == 0) {
     a.rho[k] = rho;
     a.hs[k] = h;
@@ -1014,7 +1163,7 @@ void sph_enqueue_force(SphState& s, const double* pos, const double* vel, const 
     grid_build(s, 0, ctl, st);
     k_sph_seeds<<<flat_grid(n), kFlat, 0, st>>>(view(s, 0), s.grid[0].skey, s.grid[0].mixed, s.cbrt_tab, sc,
                                                 s.seeds);
-    k_sph_dens_cell<<<1, 1, 0, st>>>(n, sc);
+    k_sph_dens_cell<<<1, kFlat, 0, st>>>(n, sc);
     grid_build(s, 1, ctl, st);
     DensArgs da;
     da.g = view(s, 1);

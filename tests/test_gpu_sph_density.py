@@ -1,0 +1,44 @@
+"""Smoothing lengths where the density's root search starts badly: sparse and crowded
+bins, duplicates, a dense core beside far outliers, few particles, other neighbour numbers.
+The bracket and bisection decide as the oracle's, so h agrees to the rounding of the seeds."""
+
+import numpy as np
+import pytest
+
+import galaxy_b200 as gb
+
+pytestmark = pytest.mark.gpu
+
+
+def _cloud(kind, n, rng):
+    if kind == "uniform":
+        return rng.random((n, 3))
+    if kind == "core":  # a dense core and outliers whose balls hold all of it
+        x = rng.normal(size=(n, 3)) * 0.01
+        x[: n // 50] = rng.normal(size=(n // 50, 3)) * 30.0
+        return x
+    if kind == "sheet":
+        x = rng.random((n, 3))
+        x[:, 2] *= 1e-3
+        return x
+    x = rng.random((n, 3))  # duplicates
+    x[n // 2:] = x[: n - n // 2]
+    return x
+
+
+@pytest.mark.parametrize("kind", ["uniform", "core", "sheet", "duplicates"])
+@pytest.mark.parametrize("n", [2, 31, 65, 700, 3000])
+@pytest.mark.parametrize("n_ngb", [12.0, 48.0, 300.0])
+def test_h_matches_oracle(oracle, kind, n, n_ngb):
+    rng = np.random.default_rng(n)
+    pos, mass = _cloud(kind, n, rng), rng.uniform(0.5, 1.0, n)
+    s = gb.GpuGravitySph(1.0, 0.01, 0.5, sph=dict(n_ngb=n_ngb))
+    ref_rho, ref_h = oracle.sph_density_adaptive(pos, mass, n_ngb=n_ngb)
+    for hint in (None, ref_h, ref_h * 1.7, ref_h * 0.2):
+        rho, h = s.density(pos, mass, hint)
+        if hint is not None:
+            ref_rho2, ref_h2 = oracle.sph_density_adaptive(pos, mass, n_ngb=n_ngb, h_init=hint)
+        else:
+            ref_rho2, ref_h2 = ref_rho, ref_h
+        assert np.allclose(h, ref_h2, rtol=1e-12, atol=0.0)
+        assert np.allclose(rho, ref_rho2, rtol=1e-11, atol=0.0)
