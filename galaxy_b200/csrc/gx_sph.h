@@ -65,6 +65,8 @@ struct SphState {
   double* rho_act = nullptr;    // the active path's persistent density scratch
   double4* sv = nullptr;   // hydro grid order: vx, vy, vz, h
   double4* sa = nullptr;   // hydro grid order: rho, P/rho^2 term, 1/(pi h^3), c_s
+  uint32_t* hcell = nullptr;  // per hydro bucket: the largest h in it, as the bits of a float
+  float* reach = nullptr;     // per hydro slot: the largest h within two cells
   SphScalars* sc = nullptr;
   SphGrid grid[3];  // occupancy, density query, hydro
   // sort scratch of the grids (one system of n_gas)
