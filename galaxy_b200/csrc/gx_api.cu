@@ -22,6 +22,7 @@
 #include "gx_kernels.h"
 #include "gx_runtime.h"
 #include "gx_sph.h"
+#include "gx_transfer.h"
 
 using namespace gx;
 
@@ -486,13 +487,18 @@ void enqueue_force(gx_handle* h, const StepBufs& b, int kick, int pending, bool 
   h->launches += 1;
 }
 
-// Wait for the stream, then turn the device error word into a status.
-int finish(gx_handle* h, bool timed) {
-  GX_CK(h, cudaStreamSynchronize(h->stream));
+// Wait for the stream, copying `outs` to the host after it, then turn the device error
+// word (copied to pinned memory in the same wait) into a status.
+int finish(gx_handle* h, bool timed, const HostPiece* outs = nullptr, int n_outs = 0) {
+  if (h->ar.b.ctl)
+    GX_CK(h, cudaMemcpyAsync(h->ctl_host, h->ar.b.ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, h->stream));
+  if (n_outs)
+    GX_CK(h, copy_out(h->device, h->stream, outs, n_outs));
+  else
+    GX_CK(h, cudaStreamSynchronize(h->stream));
   GX_CK(h, cudaGetLastError());
   if (!h->ar.b.ctl) return GX_OK;  // nothing allocated yet (empty system)
-  DevCtl ctl;
-  GX_CK(h, cudaMemcpy(&ctl, h->ar.b.ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost));
+  const DevCtl ctl = *h->ctl_host;
   if (timed) {
     cudaEventElapsedTime(&h->stats.ms_bbox_morton, h->ev[0], h->ev[1]);
     cudaEventElapsedTime(&h->stats.ms_sort, h->ev[1], h->ev[2]);
@@ -608,6 +614,7 @@ int gx_create(double g, double softening, double theta, const gx_options* opt, g
     delete h;
     return GX_ERR_CUDA;
   }
+  transfer_ref();
   *out = h;
   return GX_OK;
 }
@@ -627,6 +634,7 @@ void gx_destroy(gx_handle* h) {
     if (e) cudaEventDestroy(e);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
+  transfer_unref();
 }
 
 const char* gx_last_error(const gx_handle* h) { return h ? h->err.c_str() : global_err(); }
@@ -713,12 +721,12 @@ int gx_accelerations(gx_handle* h, size_t n, const double* pos, const double* ma
   int rc = layout(h, n, 0.0);
   if (rc) return rc;
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(b.pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, mass, n * sizeof(double)));
   enqueue_force(h, b, 0, 0, stats_on(h));
-  GX_CK(h, cudaMemcpyAsync(acc_out, b.acc, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   h->stats.n = n;
-  return finish(h, stats_on(h));
+  const HostPiece out{acc_out, b.acc, 3 * n * sizeof(double)};
+  return finish(h, stats_on(h), &out, 1);
 }
 
 int gx_accelerations_device(gx_handle* h, size_t n, const double* d_pos, const double* d_mass, double* d_acc) {
@@ -771,9 +779,9 @@ int walk_active(gx_handle* h, size_t n, size_t n_active, const uint32_t* active,
   h->launches += 1;
   launch_gather_acc(b.acc, a.active, na, a.out, h->stream);
   std::vector<double> got(3 * n_active);
-  GX_CK(h, cudaMemcpyAsync(got.data(), a.out, 3 * n_active * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   h->stats.n = n;
-  const int rc = finish(h, timed);
+  const HostPiece out{got.data(), a.out, 3 * n_active * sizeof(double)};
+  const int rc = finish(h, timed, &out, 1);
   if (rc) return rc;
   for (size_t i = 0; i < n_active; ++i)
     for (int c = 0; c < 3; ++c) acc_out[3 * (size_t)active[i] + c] = got[3 * i + c];
@@ -807,9 +815,9 @@ int gx_accelerations_active(gx_handle* h, size_t n, const double* pos, const dou
   if (rc) return rc;
   GX_CK(h, ensure_active(h, n, n_active));
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(b.pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->act.active, active, n_active * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, mass, n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->act.active, active, n_active * sizeof(uint32_t)));
   const bool timed = stats_on(h);
   enqueue_tree(h, b, 0, 0, timed);
   return walk_active(h, n, n_active, active, acc_out, timed);
@@ -826,8 +834,8 @@ int gx_rebuild_gravity_cache(gx_handle* h, size_t n, const double* pos, const do
   int rc = layout(h, n, 0.0);
   if (rc) return rc;
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(b.pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, mass, n * sizeof(double)));
   enqueue_tree(h, b, 0, 0, false);
   rc = finish(h, false);
   if (rc) return rc;
@@ -851,9 +859,9 @@ int gx_gravity_active_cached(gx_handle* h, size_t n, const double* pos, const do
   cudaSetDevice(h->device);
   GX_CK(h, ensure_active(h, n, n_active));
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(b.pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->act.active, active, n_active * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, mass, n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->act.active, active, n_active * sizeof(uint32_t)));
   // the walk's own per-step counters start at zero (the tree is not rebuilt)
   GX_CK(h, cudaMemsetAsync(b.counters, 0, kCounterWords * sizeof(uint32_t), h->stream));
   launch_refresh_leaves(b, h->stream);
@@ -876,8 +884,8 @@ int gx_potential_energy(gx_handle* h, size_t n, const double* pos, const double*
   int rc = layout(h, n, 0.0);
   if (rc) return rc;
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(b.pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, mass, n * sizeof(double)));
   const uint32_t np = potential_partials(static_cast<uint32_t>(n));
   launch_potential_f64(static_cast<uint32_t>(n), b.pos, b.mass, h->g, h->eps, h->ar.diag_partial, np, h->stream);
   std::vector<double> part(np);
@@ -901,8 +909,8 @@ int gx_direct_sum_f64(gx_handle* h, size_t n, const double* pos, const double* m
   int rc = layout(h, std::max(n, n_targets), 0.0);
   if (rc) return rc;
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(b.pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, mass, n * sizeof(double)));
   uint32_t* d_t = nullptr;
   if (targets) {
     d_t = b.keys_alt;
@@ -935,9 +943,9 @@ int upload_impl(gx_handle* h, size_t n, const double* pos, const double* vel, co
   int rc = layout(h, n, 0.0);
   if (rc) return rc;
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(b.pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(b.vel, vel, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, b.vel, vel, 3 * n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, mass, n * sizeof(double)));
   h->sph_host_hint_ngas = 0;
   if (gas && !gas->empty()) {
     // the gas map is rebuilt from the species at every upload (gpu_resident_sph.rs:170-194)
@@ -946,7 +954,7 @@ int upload_impl(gx_handle* h, size_t n, const double* pos, const double* vel, co
     if (u) {
       std::vector<double> gu(gas->size());
       for (size_t k = 0; k < gas->size(); ++k) gu[k] = u[(*gas)[k]];
-      GX_CK(h, cudaMemcpy(h->sph.gu, gu.data(), gu.size() * sizeof(double), cudaMemcpyHostToDevice));
+      GX_CK(h, copy_in(h->device, h->stream, h->sph.gu, gu.data(), gu.size() * sizeof(double)));
     }
     h->resident_gas = true;
   }
@@ -1082,7 +1090,7 @@ int gx_kdk_step_host(gx_handle* h, size_t n, double* pos, double* vel, const dou
   rc = layout(h, n, 0.0);
   if (rc) return rc;
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, mass, n * sizeof(double)));
   const size_t chunk = std::max<size_t>(size_t{1} << 16, (n + 7) / 8);
   for (size_t c0 = 0; c0 < n; c0 += chunk) {
     const long long i0 = static_cast<long long>(3 * c0);
@@ -1146,9 +1154,8 @@ int gx_snapshot(gx_handle* h, double* pos_out, double* vel_out) {
   cudaSetDevice(h->device);
   apply_pending(h);
   const size_t bytes = 3 * h->n * sizeof(double);
-  if (pos_out) GX_CK(h, cudaMemcpyAsync(pos_out, h->ar.b.pos, bytes, cudaMemcpyDeviceToHost, h->stream));
-  if (vel_out) GX_CK(h, cudaMemcpyAsync(vel_out, h->ar.b.vel, bytes, cudaMemcpyDeviceToHost, h->stream));
-  return finish(h, false);
+  const HostPiece outs[2] = {{pos_out, h->ar.b.pos, bytes}, {vel_out, h->ar.b.vel, bytes}};
+  return finish(h, false, outs, 2);
 }
 
 int gx_resident_accelerations(gx_handle* h, double* acc_out) {
@@ -1156,8 +1163,8 @@ int gx_resident_accelerations(gx_handle* h, double* acc_out) {
   if (!h->resident) return fail(h, GX_ERR_STATE, "no resident state");
   if (h->n == 0) return GX_OK;
   cudaSetDevice(h->device);
-  GX_CK(h, cudaMemcpyAsync(acc_out, h->ar.b.acc, 3 * h->n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  return finish(h, false);
+  const HostPiece out{acc_out, h->ar.b.acc, 3 * h->n * sizeof(double)};
+  return finish(h, false, &out, 1);
 }
 
 int gx_time(const gx_handle* h, double* t_out) {
@@ -1344,7 +1351,7 @@ int gx_stage_morton(gx_handle* h, size_t n, const double* pos, uint32_t* lanes_o
   int rc = layout(h, n, 0.0);
   if (rc) return rc;
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(b.pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
   GX_CK(h, cudaMemsetAsync(b.zero_begin, 0, b.zero_bytes, h->stream));
   launch_kick_drift_bbox(b, 0, 0, h->stream);
   // Lanes (3n u32) are staged in the walk records, unused by this stage.
@@ -1406,8 +1413,8 @@ int gx_stage_build(gx_handle* h, size_t n, const uint32_t* sorted_codes, const d
   for (size_t i = 0; i < n; ++i) iota[i] = static_cast<uint32_t>(i);
   GX_CK(h, cudaMemcpyAsync(b.codes, sorted_codes, n * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
   GX_CK(h, cudaMemcpyAsync(b.order, iota.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(b.pos, sorted_pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, sorted_mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, sorted_pos, 3 * n * sizeof(double)));
+  GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, sorted_mass, n * sizeof(double)));
   const int quad = h->opt.multipole == GX_MULTIPOLE_QUAD && h->opt.precision != GX_PREC_F64;
   GX_CK(h, cudaMemsetAsync(b.bounds, 0, sizeof(Bounds), h->stream));  // no Morton stage here
   launch_build(b, quad, h->stream);
@@ -1507,9 +1514,9 @@ int host_sph_setup(gx_handle* h, size_t n, const double* pos, const double* vel,
   int rc = layout(h, n, 0.0);
   if (rc) return rc;
   StepBufs& b = h->ar.b;
-  GX_CK(h, cudaMemcpyAsync(b.pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  if (vel) GX_CK(h, cudaMemcpyAsync(b.vel, vel, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  if (mass) GX_CK(h, cudaMemcpyAsync(h->ar.mass_rw, mass, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
+  if (vel) GX_CK(h, copy_in(h->device, h->stream, b.vel, vel, 3 * n * sizeof(double)));
+  if (mass) GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, mass, n * sizeof(double)));
   if (gas) {
     h->sph.gas_idx_host = *gas;
   } else {
@@ -1607,9 +1614,8 @@ int gx_snapshot_gas_density(gx_handle* h, uint32_t* gas_idx_out, double* rho_out
   cudaSetDevice(h->device);
   const size_t ng = h->sph.n_gas;
   if (gas_idx_out) std::memcpy(gas_idx_out, h->sph.gas_idx_host.data(), ng * sizeof(uint32_t));
-  if (rho_out) GX_CK(h, cudaMemcpyAsync(rho_out, h->sph.rho, ng * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  if (h_out) GX_CK(h, cudaMemcpyAsync(h_out, h->sph.hs, ng * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  return finish(h, false);
+  const HostPiece outs[2] = {{rho_out, h->sph.rho, ng * sizeof(double)}, {h_out, h->sph.hs, ng * sizeof(double)}};
+  return finish(h, false, outs, 2);
 }
 
 int gx_snapshot_gas_accel(gx_handle* h, double* acc_out, double* dudt_out) {
@@ -1689,19 +1695,15 @@ int gx_sph_accel_and_dudt(gx_handle* h, size_t n, const double* pos, const doubl
     if (u) {
       std::vector<double> gu(gas.size());
       for (size_t k = 0; k < gas.size(); ++k) gu[k] = u[gas[k]];
-      GX_CK(h, cudaMemcpy(h->sph.gu, gu.data(), gu.size() * sizeof(double), cudaMemcpyHostToDevice));
+      GX_CK(h, copy_in(h->device, h->stream, h->sph.gu, gu.data(), gu.size() * sizeof(double)));
     }
     sph_enqueue_force(h->sph, b.pos, b.vel, b.mass, b.acc, true, true, b.ctl, h->stream);
   }
-  GX_CK(h, cudaMemcpyAsync(acc_out, b.acc, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  std::vector<double> gdudt;
-  if (dudt_out && !gas.empty()) {
-    gdudt.resize(gas.size());
-    GX_CK(h, cudaMemcpyAsync(gdudt.data(), h->sph.dudt, gas.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                             h->stream));
-  }
+  std::vector<double> gdudt(dudt_out ? gas.size() : 0);
   h->stats.n = n;
-  rc = finish(h, stats_on(h));
+  const HostPiece outs[2] = {{acc_out, b.acc, 3 * n * sizeof(double)},
+                             {gdudt.data(), h->sph.dudt, gdudt.size() * sizeof(double)}};
+  rc = finish(h, stats_on(h), outs, 2);
   if (rc != GX_OK) return rc;
   h->sph_host_hint_ngas = gas.size();
   if (dudt_out) {
@@ -1765,7 +1767,7 @@ int gx_sph_accel_and_dudt_active(gx_handle* h, size_t n, const double* pos, cons
     if (u) {
       std::vector<double> gu(ng);
       for (size_t k = 0; k < ng; ++k) gu[k] = u[gas[k]];
-      GX_CK(h, cudaMemcpy(h->sph.gu, gu.data(), ng * sizeof(double), cudaMemcpyHostToDevice));
+      GX_CK(h, copy_in(h->device, h->stream, h->sph.gu, gu.data(), ng * sizeof(double)));
     }
     // the density pass writes the refreshed rows over the active path's rho scratch
     if (rho_set)
@@ -1860,7 +1862,7 @@ int gx_sph_max_stable_dt(gx_handle* h, size_t n, const double* pos, const double
   if (u) {
     std::vector<double> gu(ng);
     for (size_t k = 0; k < ng; ++k) gu[k] = u[gas[k]];
-    GX_CK(h, cudaMemcpy(h->sph.gu, gu.data(), ng * sizeof(double), cudaMemcpyHostToDevice));
+    GX_CK(h, copy_in(h->device, h->stream, h->sph.gu, gu.data(), ng * sizeof(double)));
   }
   const StepBufs& b = h->ar.b;
   sph_enqueue_force(h->sph, b.pos, b.vel, b.mass, nullptr, true, false, b.ctl, h->stream);

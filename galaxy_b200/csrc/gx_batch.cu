@@ -16,6 +16,7 @@
 #include "gx_kernels.h"
 #include "gx_runtime.h"
 #include "gx_snapshot.h"
+#include "gx_transfer.h"
 
 using namespace gx;
 
@@ -294,6 +295,7 @@ int gx_batch_create(size_t budget_bytes, const gx_options* opt, gx_batch** out) 
     delete bt;
     return GX_ERR_CUDA;
   }
+  transfer_ref();
   *out = bt;
   return GX_OK;
 }
@@ -308,6 +310,7 @@ void gx_batch_destroy(gx_batch* bt) {
   if (bt->e1) cudaEventDestroy(bt->e1);
   if (bt->stream) cudaStreamDestroy(bt->stream);
   delete bt;
+  transfer_unref();
 }
 
 const char* gx_batch_last_error(const gx_batch* bt) { return bt ? bt->err.c_str() : global_err(); }
@@ -336,9 +339,9 @@ int gx_system_add(gx_batch* bt, size_t n, const double* pos, const double* vel, 
   if (rc) return rc;
   StepBufs& b = bt->ar.b;
   const size_t off = bt->total;
-  GB_CK(bt, cudaMemcpyAsync(b.pos + 3 * off, pos, 3 * n * 8, cudaMemcpyHostToDevice, bt->stream));
-  GB_CK(bt, cudaMemcpyAsync(b.vel + 3 * off, vel, 3 * n * 8, cudaMemcpyHostToDevice, bt->stream));
-  GB_CK(bt, cudaMemcpyAsync(bt->ar.mass_rw + off, mass, n * 8, cudaMemcpyHostToDevice, bt->stream));
+  GB_CK(bt, copy_in(bt->device, bt->stream, b.pos + 3 * off, pos, 3 * n * 8));
+  GB_CK(bt, copy_in(bt->device, bt->stream, b.vel + 3 * off, vel, 3 * n * 8));
+  GB_CK(bt, copy_in(bt->device, bt->stream, bt->ar.mass_rw + off, mass, n * 8));
   GB_CK(bt, cudaMemsetAsync(b.acc + 3 * off, 0, 3 * n * 8, bt->stream));
   BatchSys s{};
   s.id = bt->next_id++;
@@ -521,21 +524,16 @@ int gx_system_snapshot(gx_batch* bt, uint64_t id, double* pos_out, double* vel_o
   cudaSetDevice(bt->device);
   const BatchSys& s = bt->systems[i];
   const StepBufs& b = bt->ar.b;
-  std::vector<double> vel(3 * (size_t)s.n), acc(3 * (size_t)s.n);
-  if (pos_out) GB_CK(bt, cudaMemcpyAsync(pos_out, b.pos + 3 * (size_t)s.off, 3 * (size_t)s.n * 8, cudaMemcpyDeviceToHost, bt->stream));
-  GB_CK(bt, cudaMemcpyAsync(vel.data(), b.vel + 3 * (size_t)s.off, 3 * (size_t)s.n * 8, cudaMemcpyDeviceToHost, bt->stream));
-  if (s.pending)
-    GB_CK(bt, cudaMemcpyAsync(acc.data(), b.acc + 3 * (size_t)s.off, 3 * (size_t)s.n * 8, cudaMemcpyDeviceToHost, bt->stream));
-  GB_CK(bt, cudaStreamSynchronize(bt->stream));
-  if (s.pending) {
-    // The owed closing half kick, applied to the copy (v + a*(0.5 dt), one rounding each).
-    volatile double h = 0.5 * s.dt;
-    for (size_t j = 0; j < vel.size(); ++j) {
-      volatile double t = acc[j] * h;
-      vel[j] = vel[j] + t;
-    }
-  }
-  if (vel_out) memcpy(vel_out, vel.data(), vel.size() * sizeof(double));
+  // pos and vel with the owed closing half kick (v + a*(0.5 dt), one rounding each), staged
+  // in the system's walk records (80 bytes a particle, rebuilt by the next step)
+  double* stage = reinterpret_cast<double*>(b.pairs + 5 * (size_t)s.off);
+  const uint32_t grid = std::max(1u, std::min((s.n + 255u) / 256u, 148u * 8u));
+  k_stage_snapshot<<<grid, 256, 0, bt->stream>>>(s.off, s.n, b.pos, b.vel, b.acc, b.mass, s.pending ? 1 : 0, s.dt,
+                                                 stage);
+  GB_CK(bt, cudaGetLastError());
+  const size_t bytes = 3 * (size_t)s.n * 8;
+  const HostPiece outs[2] = {{pos_out, stage, bytes}, {vel_out, stage + 3 * (size_t)s.n, bytes}};
+  GB_CK(bt, copy_out(bt->device, bt->stream, outs, 2));
   if (time_out) *time_out = s.time;
   return GX_OK;
 }

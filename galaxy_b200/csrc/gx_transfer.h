@@ -1,0 +1,26 @@
+// gx_transfer.h -- host <-> device copies of callers' arrays (gx_transfer.cpp).
+#pragma once
+
+#include <cstddef>
+#include <cuda_runtime.h>
+
+namespace gx {
+
+struct HostPiece {
+  void* host;       // null: skipped
+  const void* dev;
+  size_t bytes;
+};
+
+// dst (device) <- src (host), in order on st. src has been read when it returns, unless it
+// is pinned (then it must stay until the copy has run, as for cudaMemcpyAsync). The device
+// is the current one.
+cudaError_t copy_in(int device, cudaStream_t st, void* dst, const void* src, size_t bytes);
+// The pieces' device memory, after the work enqueued on st, to the host: complete, and the
+// stream idle, when it returns.
+cudaError_t copy_out(int device, cudaStream_t st, const HostPiece* pieces, int count);
+// Every handle and batch holds a reference; the last one frees the idle staging buffers.
+void transfer_ref();
+void transfer_unref();
+
+}  // namespace gx
