@@ -39,7 +39,16 @@ __device__ __forceinline__ void block_bbox_commit(double v[6], unsigned long lon
 
 }  // namespace
 
-// One CTA per tile. kick: apply the (deferred closing +) opening half kick and the
+// The part of tile blockIdx.x / split that this block takes, [begin, end).
+__device__ __forceinline__ TileDesc tile_part(const TileDesc* __restrict__ tiles, int split) {
+  TileDesc t = tiles[blockIdx.x / split];
+  const uint32_t len = kTile / split;
+  t.begin += (blockIdx.x % split) * len;
+  t.end = min(t.end, t.begin + len);
+  return t;
+}
+
+// `split` CTAs per tile. kick: apply the (deferred closing +) opening half kick and the
 // drift before reducing the bounding box of the new positions.
 //   pending:  v += a*h   (closing half kick of the previous step, kept separate)
 //   always:   v += a*h ; x += v*dt        with h = 0.5*dt     (integrator.rs:59-67)
@@ -47,8 +56,9 @@ __global__ void __launch_bounds__(kTileThreads) k_kick_drift_bbox(const TileDesc
                                                                   const SysDesc* __restrict__ sys,
                                                                   double* __restrict__ pos, double* __restrict__ vel,
                                                                   const double* __restrict__ acc, int kick,
-                                                                  int pending, unsigned long long* __restrict__ enc) {
-  const TileDesc t = tiles[blockIdx.x];
+                                                                  int pending, unsigned long long* __restrict__ enc,
+                                                                  int split) {
+  const TileDesc t = tile_part(tiles, split);
   const SysDesc s = sys[t.sys];
   const double dt = s.dt;
   const double h = dmul(0.5, dt);
@@ -84,8 +94,8 @@ __global__ void __launch_bounds__(kTileThreads) k_kick_drift_bbox(const TileDesc
 // Closing half kick only (applied before a snapshot when one is pending).
 __global__ void __launch_bounds__(kTileThreads) k_kick_half(const TileDesc* __restrict__ tiles,
                                                             const SysDesc* __restrict__ sys, double* __restrict__ vel,
-                                                            const double* __restrict__ acc) {
-  const TileDesc t = tiles[blockIdx.x];
+                                                            const double* __restrict__ acc, int split) {
+  const TileDesc t = tile_part(tiles, split);
   const double h = dmul(0.5, sys[t.sys].dt);
   for (uint32_t i = t.begin + threadIdx.x; i < t.end; i += kTileThreads) {
 #pragma unroll
@@ -119,7 +129,7 @@ __device__ __forceinline__ void make_bounds(const unsigned long long* e, Bounds&
   b.tiny2 = static_cast<float>(t * t);
 }
 
-// One CTA per tile: Morton code of every particle of the tile (original order) and
+// `split` CTAs per tile: Morton code of every particle of the tile (original order) and
 // the tile's contribution to the per-system digit histograms of all radix passes
 // (4 for 30-bit keys, 8 for 63-bit). The tile's system cube is rebuilt from the
 // reduced lo/hi by every CTA (a few flops), and the system's first tile publishes it.
@@ -130,16 +140,16 @@ __global__ void __launch_bounds__(kTileThreads) k_morton_hist(const TileDesc* __
                                                               const SysDesc* __restrict__ sys,
                                                               Bounds* __restrict__ bounds, uint32_t* __restrict__ codes,
                                                               uint32_t* __restrict__ lanes_out,
-                                                              uint32_t* __restrict__ hist) {
+                                                              uint32_t* __restrict__ hist, int split) {
   constexpr int BINS = 1 << BITS;
   constexpr int P = K64 ? (63 + BITS - 1) / BITS : (30 + BITS - 1) / BITS;
   __shared__ uint32_t sh[P][BINS];
   __shared__ Bounds sb;
-  const TileDesc t = tiles[blockIdx.x];
+  const TileDesc t = tile_part(tiles, split);
   for (int i = threadIdx.x; i < P * BINS; i += kTileThreads) (&sh[0][0])[i] = 0;
   if (threadIdx.x == 0) {
     make_bounds(enc + 6 * (size_t)t.sys, sb);
-    if (sys[t.sys].first_tile == blockIdx.x) bounds[t.sys] = sb;
+    if (sys[t.sys].first_tile * split == blockIdx.x) bounds[t.sys] = sb;
   }
   __syncthreads();
   const double bx = sb.bmin[0], by = sb.bmin[1], bz = sb.bmin[2];
@@ -175,24 +185,40 @@ __global__ void __launch_bounds__(kTileThreads) k_morton_hist(const TileDesc* __
 }
 
 // ---- host launchers ---------------------------------------------------------------
+namespace {
+
+// CTAs per tile of the streaming kernels: a tile a CTA leaves most SMs idle, and 16 particles
+// a thread one after another, until there are a few tiles per SM. The histogram kernel
+// pays one merge of its bins per CTA, so it splits less.
+// Measured (kick + bbox and Morton together, us): 4,096 particles 36 -> 18, 65,536 36 ->
+// 20, 200,003 38 -> 23, 600,000 42 -> 37.
+int stream_split(uint32_t ntiles) { return ntiles <= 74 ? 16 : ntiles <= 296 ? 4 : 1; }
+int hist_split(uint32_t ntiles) { return ntiles <= 37 ? 8 : ntiles <= 148 ? 4 : 1; }
+
+}  // namespace
+
 void launch_kick_drift_bbox(const StepBufs& b, int kick, int pending, cudaStream_t st) {
-  k_kick_drift_bbox<<<b.ntiles, kTileThreads, 0, st>>>(b.tiles, b.sys, b.pos, b.vel, b.acc, kick, pending, b.bbox_enc);
+  const int split = stream_split(b.ntiles);
+  k_kick_drift_bbox<<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.sys, b.pos, b.vel, b.acc, kick, pending,
+                                                               b.bbox_enc, split);
 }
 
 void launch_kick_half(const StepBufs& b, cudaStream_t st) {
-  k_kick_half<<<b.ntiles, kTileThreads, 0, st>>>(b.tiles, b.sys, b.vel, b.acc);
+  const int split = stream_split(b.ntiles);
+  k_kick_half<<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.sys, b.vel, b.acc, split);
 }
 
 void launch_morton_hist(const StepBufs& b, uint32_t* lanes_out, cudaStream_t st) {
+  const int split = hist_split(b.ntiles);
   if (b.key64)
-    k_morton_hist<true, kRadixBits><<<b.ntiles, kTileThreads, 0, st>>>(b.tiles, b.pos, b.bbox_enc, b.sys, b.bounds,
-                                                                        b.codes, nullptr, b.hist);
+    k_morton_hist<true, kRadixBits><<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.pos, b.bbox_enc, b.sys, b.bounds,
+                                                                        b.codes, nullptr, b.hist, split);
   else if (b.radix_bits == kRadixBitsWide)
-    k_morton_hist<false, kRadixBitsWide><<<b.ntiles, kTileThreads, 0, st>>>(b.tiles, b.pos, b.bbox_enc, b.sys,
-                                                                             b.bounds, b.codes, lanes_out, b.hist);
+    k_morton_hist<false, kRadixBitsWide><<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.pos, b.bbox_enc, b.sys,
+                                                                             b.bounds, b.codes, lanes_out, b.hist, split);
   else
-    k_morton_hist<false, kRadixBits><<<b.ntiles, kTileThreads, 0, st>>>(b.tiles, b.pos, b.bbox_enc, b.sys, b.bounds,
-                                                                         b.codes, lanes_out, b.hist);
+    k_morton_hist<false, kRadixBits><<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.pos, b.bbox_enc, b.sys, b.bounds,
+                                                                         b.codes, lanes_out, b.hist, split);
 }
 
 }  // namespace gx
