@@ -76,6 +76,7 @@ void prepare_device(int dev) {
   if (dev < 0 || dev >= 64 || (done >> dev) & 1u) return;
   walk_prepare();
   build_prepare();
+  small_sort_prepare();
   done |= 1ull << dev;
 }
 
@@ -451,18 +452,24 @@ int layout(gx_handle* h, size_t n, double dt) {
 // Enqueue bbox (+kick/drift) -> Morton -> sort -> build on b.
 void enqueue_tree(gx_handle* h, const StepBufs& b, int kick, int pending, bool timed) {
   cudaStream_t st = h->stream;
+  // One block sorts what fits its shared memory (codes included, so the Morton stage's time
+  // counts as the sort's); a fixed 10-bit digit width keeps the pass kernels.
+  const bool small = b.n <= small_sort_max() && b.radix_bits == kRadixBits;
   ++h->tree_gen;
   if (timed) cudaEventRecord(h->ev[0], st);
   {
     NvtxRange r("gx.kick_drift_bbox_morton");
     cudaMemsetAsync(b.zero_begin, 0, b.zero_bytes, st);
     launch_kick_drift_bbox(b, kick, pending, st);
-    launch_morton_hist(b, nullptr, st);
+    if (!small) launch_morton_hist(b, nullptr, st);
   }
   if (timed) cudaEventRecord(h->ev[1], st);
   {
     NvtxRange r("gx.sort");
-    launch_sort(b, st);
+    if (small)
+      launch_small_sort(b, st);
+    else
+      launch_sort(b, st);
   }
   if (timed) cudaEventRecord(h->ev[2], st);
   {

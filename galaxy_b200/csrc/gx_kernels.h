@@ -97,6 +97,11 @@ void launch_sort_passes(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* v
 // per-system digit histograms of b.codes (when codes come from the host)
 void launch_code_hist(const StepBufs& b, cudaStream_t st);
 // gx_build.cu: gather leaves + bottom-up Karras build and aggregation
+// Morton codes and sort of one system of at most small_sort_max() particles in one
+// launch (8-bit digits); small_sort_prepare once per device.
+uint32_t small_sort_max();
+void small_sort_prepare();
+void launch_small_sort(const StepBufs& b, cudaStream_t st);
 void launch_build(const StepBufs& b, int quad, cudaStream_t st);
 // Per-device set-up of the build kernels (their dynamic shared-memory limit); call with the
 // device current, before any stream capture.

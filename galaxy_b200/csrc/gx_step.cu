@@ -184,8 +184,149 @@ __global__ void __launch_bounds__(kTileThreads) k_morton_hist(const TileDesc* __
   }
 }
 
+namespace {
+
+constexpr int kSmallThreads = 1024, kSmallWarps = kSmallThreads / 32;
+
+// Shared memory of the one-block Morton sort.
+template <typename K, int ITEMS>
+struct SmallSmem {
+  K key[kSmallThreads * ITEMS];
+  uint16_t val[kSmallThreads * ITEMS];  // local particle index
+  uint32_t cnt[kSmallWarps][kRadixBins];  // digit counts, then offsets, per warp
+  uint32_t part[kSmallThreads / kRadixBins][kRadixBins];
+  uint32_t start[kRadixBins];
+  uint32_t wsum[kRadixBins / 32];
+  Bounds bounds;
+};
+
+}  // namespace
+
+// Morton codes and the whole stable sort of one small system in one block: every digit pass
+// stays in registers and shared memory, in place of the code kernel and four (eight)
+// launches whose look-back, histograms and scattered writes take 7 to 10 us each whatever
+// N is. Keys are ranked as in k_onesweep (a warp owns 32 ITEMS consecutive keys, peers from
+// __match_any_sync), so the permutation is the same. Bound by the ranking's chain of ITEMS
+// steps a pass, so it stops at a tile: kick, codes and sort together 512 particles 45 -> 24
+// us, 4,096 63 -> 41 (63-bit keys 107 -> 67); 8,192 would gain nothing (62 and 59, 113 and
+// 110), 16,384 lose (57 and 81).
+template <typename K, int ITEMS>
+__global__ void __launch_bounds__(kSmallThreads) k_small_sort(uint32_t n, const double* __restrict__ pos,
+                                                              const unsigned long long* __restrict__ enc,
+                                                              Bounds* __restrict__ bounds, K* __restrict__ codes,
+                                                              uint32_t* __restrict__ order) {
+  extern __shared__ __align__(16) unsigned char s_small_raw[];
+  SmallSmem<K, ITEMS>& S = *reinterpret_cast<SmallSmem<K, ITEMS>*>(s_small_raw);
+  constexpr int PASSES = sizeof(K) == 8 ? kRadixPasses63 : kRadixPasses;
+  constexpr int PARTS = kSmallThreads / kRadixBins;  // threads a digit
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  if (tid == 0) {
+    make_bounds(enc, S.bounds);
+    bounds[0] = S.bounds;
+  }
+  __syncthreads();
+  const double bx = S.bounds.bmin[0], by = S.bounds.bmin[1], bz = S.bounds.bmin[2];
+  const double scale = sizeof(K) == 8 ? S.bounds.scale63 : S.bounds.scale;
+  K key[ITEMS];
+  uint32_t val[ITEMS], rank[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const uint32_t i = warp * (32 * ITEMS) + 32 * j + lane;
+    val[j] = i;
+    key[j] = ~K(0);  // past the end: the largest digits, and last among equals
+    if (i < n) {
+      const double vx = dmul(dsub(pos[3 * (size_t)i + 0], bx), scale);
+      const double vy = dmul(dsub(pos[3 * (size_t)i + 1], by), scale);
+      const double vz = dmul(dsub(pos[3 * (size_t)i + 2], bz), scale);
+      if (sizeof(K) == 8)
+        key[j] = static_cast<K>(morton3_63(quantize_lane21(vx), quantize_lane21(vy), quantize_lane21(vz)));
+      else
+        key[j] = static_cast<K>(morton3(quantize_lane(vx), quantize_lane(vy), quantize_lane(vz)));
+    }
+  }
+  for (int pass = 0; pass < PASSES; ++pass) {
+    const int shift = pass * kRadixBits;
+    for (int i = tid; i < kSmallWarps * kRadixBins; i += kSmallThreads) (&S.cnt[0][0])[i] = 0u;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t d = static_cast<uint32_t>(key[j] >> shift) & (kRadixBins - 1);
+      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t before = S.cnt[warp][d];
+      rank[j] = before + __popc(peers & lt);
+      __syncwarp();
+      if (lane == 31 - __clz(peers)) S.cnt[warp][d] = before + __popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    // digit totals and the warps' offsets within a digit, PARTS threads a digit
+    const uint32_t d = tid & (kRadixBins - 1), part = tid / kRadixBins;
+    constexpr int WP = kSmallWarps / PARTS;
+    uint32_t sum = 0;
+#pragma unroll
+    for (int w = 0; w < WP; ++w) {
+      const uint32_t c = S.cnt[part * WP + w][d];
+      S.cnt[part * WP + w][d] = sum;
+      sum += c;
+    }
+    S.part[part][d] = sum;
+    __syncthreads();
+    uint32_t below = 0, incl = 0, total = 0;
+    if (tid < kRadixBins) {
+#pragma unroll
+      for (int p = 0; p < PARTS; ++p) {
+        const uint32_t c = S.part[p][d];
+        S.part[p][d] = total;
+        total += c;
+      }
+      incl = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) S.wsum[warp] = incl;
+    }
+    __syncthreads();
+    if (tid < kRadixBins) {
+      for (int w = 0; w < warp; ++w) below += S.wsum[w];
+      S.start[d] = below + incl - total;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t dj = static_cast<uint32_t>(key[j] >> shift) & (kRadixBins - 1);
+      const uint32_t at = S.start[dj] + S.part[warp / WP][dj] + S.cnt[warp][dj] + rank[j];
+      S.key[at] = key[j];
+      S.val[at] = static_cast<uint16_t>(val[j]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t i = warp * (32 * ITEMS) + 32 * j + lane;
+      key[j] = S.key[i];
+      val[j] = S.val[i];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const uint32_t i = warp * (32 * ITEMS) + 32 * j + lane;
+    if (i < n) {
+      codes[i] = key[j];
+      order[i] = val[j];
+    }
+  }
+}
+
 // ---- host launchers ---------------------------------------------------------------
 namespace {
+
+template <typename K, int ITEMS>
+void run_small(const StepBufs& b, cudaStream_t st) {
+  k_small_sort<K, ITEMS><<<1, kSmallThreads, sizeof(SmallSmem<K, ITEMS>), st>>>(
+      b.n, b.pos, b.bbox_enc, b.bounds, reinterpret_cast<K*>(b.codes), b.order);
+}
 
 // CTAs per tile of the streaming kernels: a tile a CTA leaves most SMs idle, and 16 particles
 // a thread one after another, until there are a few tiles per SM. The histogram kernel
@@ -201,6 +342,26 @@ void launch_kick_drift_bbox(const StepBufs& b, int kick, int pending, cudaStream
   const int split = stream_split(b.ntiles);
   k_kick_drift_bbox<<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.sys, b.pos, b.vel, b.acc, kick, pending,
                                                                b.bbox_enc, split);
+}
+
+uint32_t small_sort_max() { return kTile; }
+
+void small_sort_prepare() {
+  auto set = [](auto kern, size_t bytes) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  };
+  set(k_small_sort<uint32_t, 1>, sizeof(SmallSmem<uint32_t, 1>));
+  set(k_small_sort<uint32_t, 4>, sizeof(SmallSmem<uint32_t, 4>));
+  set(k_small_sort<uint64_t, 1>, sizeof(SmallSmem<uint64_t, 1>));
+  set(k_small_sort<uint64_t, 4>, sizeof(SmallSmem<uint64_t, 4>));
+}
+
+void launch_small_sort(const StepBufs& b, cudaStream_t st) {
+  const bool one = b.n <= kSmallThreads;  // a key a thread, else four
+  if (b.key64)
+    one ? run_small<uint64_t, 1>(b, st) : run_small<uint64_t, 4>(b, st);
+  else
+    one ? run_small<uint32_t, 1>(b, st) : run_small<uint32_t, 4>(b, st);
 }
 
 void launch_kick_half(const StepBufs& b, cudaStream_t st) {
