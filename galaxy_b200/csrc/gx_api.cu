@@ -1424,6 +1424,7 @@ int gx_stage_build(gx_handle* h, size_t n, const uint32_t* sorted_codes, const d
   GX_CK(h, copy_in(h->device, h->stream, h->ar.mass_rw, sorted_mass, n * sizeof(double)));
   const int quad = h->opt.multipole == GX_MULTIPOLE_QUAD && h->opt.precision != GX_PREC_F64;
   GX_CK(h, cudaMemsetAsync(b.bounds, 0, sizeof(Bounds), h->stream));  // no Morton stage here
+  GX_CK(h, cudaMemsetAsync(b.slots, 0xFF, n * sizeof(unsigned long long), h->stream));  // nor the kick's arming
   launch_build(b, quad, h->stream);
   std::vector<uint2> kids(n > 1 ? n - 1 : 1);
   std::vector<Agg64> agg(n > 1 ? n - 1 : 1);

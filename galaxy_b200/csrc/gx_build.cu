@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(kBuildLeaves, (QUAD ? 2 : 3) * (256 / kBuildLe
                                                               const uint32_t* __restrict__ order,
                                                               const double* __restrict__ pos,
                                                               const double* __restrict__ mass, StepBufs b) {
+  step_kernel_begin();
   extern __shared__ __align__(16) unsigned char s_build_raw[];
   BuildSmem<QUAD>& S = *reinterpret_cast<BuildSmem<QUAD>*>(s_build_raw);
   // block j covers leaves [L (j % B), L (j % B) + L) of tile j / B (L = kBuildLeaves, B = kTile / L)
@@ -605,6 +606,7 @@ template <bool QUAD, typename K>
 __global__ void __launch_bounds__(kTileThreads) k_build_top(const TileDesc* __restrict__ tiles,
                                                             const SysDesc* __restrict__ sys, uint32_t n_total,
                                                             const K* __restrict__ codes, StepBufs b) {
+  step_kernel_begin();
   const uint32_t blk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // pass-1 block of this warp
   if (blk >= b.ntiles * kBuildBlocksPerTile) return;
   const TileDesc t = tiles[blk / kBuildBlocksPerTile];
@@ -728,11 +730,11 @@ namespace {
 template <bool QUAD, typename K>
 void launch_build_t(const StepBufs& b, const K* codes, cudaStream_t st) {
   const uint32_t blocks1 = b.ntiles * kBuildBlocksPerTile;
-  k_build_local<QUAD, K><<<blocks1, kBuildLeaves, sizeof(BuildSmem<QUAD>), st>>>(b.tiles, b.sys, b.n, codes, b.order,
-                                                                                 b.pos, b.mass, b);
+  launch_after(b.ntiles, k_build_local<QUAD, K>, blocks1, kBuildLeaves, sizeof(BuildSmem<QUAD>), st, b.tiles, b.sys, b.n, codes,
+               b.order, b.pos, b.mass, b);
   // one warp per block of pass 1 (its tops: a few each)
   const uint32_t blocks2 = (blocks1 * 32 + kTileThreads - 1) / kTileThreads;
-  k_build_top<QUAD, K><<<blocks2, kTileThreads, 0, st>>>(b.tiles, b.sys, b.n, codes, b);
+  launch_after(b.ntiles, k_build_top<QUAD, K>, blocks2, kTileThreads, 0, st, b.tiles, b.sys, b.n, codes, b);
 }
 
 }  // namespace
@@ -750,9 +752,6 @@ void build_prepare() {
 }
 
 void launch_build(const StepBufs& b, int quad, cudaStream_t st) {
-  // Every split's global rendezvous slot starts empty (one memset instead of a re-arming
-  // atomic per fold, which the next level's release would have to wait for).
-  cudaMemsetAsync(b.slots, 0xFF, static_cast<size_t>(b.n) * sizeof(unsigned long long), st);
   const uint64_t* c64 = reinterpret_cast<const uint64_t*>(b.codes);
   if (b.key64) {
     if (quad)

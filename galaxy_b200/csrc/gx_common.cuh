@@ -116,6 +116,15 @@ static_assert(kWalkItemCounter < kCounterWords, "the walk's counter is in the bl
 // has at most 30 + 32 (30-bit codes) or 63 + 32 (63-bit codes) internal levels.
 constexpr int kMaxDepth = 100;
 
+// The kernels of a step are launched so that each may be scheduled while the one before it
+// drains (launch_after in gx_kernels.h): every thread first lets the next kernel be scheduled
+// and then waits until the one before has completed and its writes are visible, ahead of
+// any access to global memory. Without that launch attribute both are no-ops.
+__device__ __forceinline__ void step_kernel_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 struct TileDesc {
   uint32_t sys, begin, end, pad;
 };

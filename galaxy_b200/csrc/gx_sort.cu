@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kTileThreads) k_onesweep(int pass, const K* __
   __shared__ uint32_t s_scan[kWarps];
   __shared__ uint32_t s_tile;
 
+  step_kernel_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int shift = pass * BITS;
   if (threadIdx.x == 0) s_tile = atomicAdd(&counters[pass], 1u);
@@ -247,8 +248,8 @@ void run_passes(int passes, const K* keys_in, K* keys_out, uint32_t* vals_out, K
     else
       kout = (p % 2 == 0) ? keys_tmp : keys_tmp2;
     uint32_t* vout = ((passes - 1 - p) % 2 == 0) ? vals_out : vals_tmp;
-    k_onesweep<K, BITS><<<ntiles, kTileThreads, onesweep_smem<K>(), st>>>(p, kin, vin, kout, vout, tiles, sys, hist,
-                                                                           status, counters, ntiles, ctl);
+    launch_after(ntiles, k_onesweep<K, BITS>, ntiles, kTileThreads, onesweep_smem<K>(), st, p, kin, vin, kout, vout, tiles, sys,
+                 hist, status, counters, ntiles, ctl);
     kin = kout;
     vin = vout;
   }

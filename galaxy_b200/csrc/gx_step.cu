@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(kTileThreads) k_kick_drift_bbox(const TileDesc
                                                                   double* __restrict__ pos, double* __restrict__ vel,
                                                                   const double* __restrict__ acc, int kick,
                                                                   int pending, unsigned long long* __restrict__ enc,
-                                                                  int split) {
+                                                                  unsigned long long* __restrict__ slots, int split) {
   const TileDesc t = tile_part(tiles, split);
   const SysDesc s = sys[t.sys];
   const double dt = s.dt;
@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(kTileThreads) k_kick_drift_bbox(const TileDesc
 #pragma unroll
   for (int c = 0; c < 6; ++c) v6[c] = -INFINITY;
   for (uint32_t i = t.begin + threadIdx.x; i < t.end; i += kTileThreads) {
+    slots[i] = kEmptySlot;  // the build's exchange words, armed here instead of by a memset
     double p[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) p[c] = pos[3 * (size_t)i + c];
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(kTileThreads) k_morton_hist(const TileDesc* __
                                                               Bounds* __restrict__ bounds, uint32_t* __restrict__ codes,
                                                               uint32_t* __restrict__ lanes_out,
                                                               uint32_t* __restrict__ hist, int split) {
+  step_kernel_begin();
   constexpr int BINS = 1 << BITS;
   constexpr int P = K64 ? (63 + BITS - 1) / BITS : (30 + BITS - 1) / BITS;
   __shared__ uint32_t sh[P][BINS];
@@ -215,6 +217,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_sort(uint32_t n, const 
                                                               const unsigned long long* __restrict__ enc,
                                                               Bounds* __restrict__ bounds, K* __restrict__ codes,
                                                               uint32_t* __restrict__ order) {
+  step_kernel_begin();
   extern __shared__ __align__(16) unsigned char s_small_raw[];
   SmallSmem<K, ITEMS>& S = *reinterpret_cast<SmallSmem<K, ITEMS>*>(s_small_raw);
   constexpr int PASSES = sizeof(K) == 8 ? kRadixPasses63 : kRadixPasses;
@@ -324,8 +327,8 @@ namespace {
 
 template <typename K, int ITEMS>
 void run_small(const StepBufs& b, cudaStream_t st) {
-  k_small_sort<K, ITEMS><<<1, kSmallThreads, sizeof(SmallSmem<K, ITEMS>), st>>>(
-      b.n, b.pos, b.bbox_enc, b.bounds, reinterpret_cast<K*>(b.codes), b.order);
+  launch_after(b.ntiles, k_small_sort<K, ITEMS>, 1, kSmallThreads, sizeof(SmallSmem<K, ITEMS>), st, b.n, b.pos, b.bbox_enc,
+               b.bounds, reinterpret_cast<K*>(b.codes), b.order);
 }
 
 // CTAs per tile of the streaming kernels: a tile a CTA leaves most SMs idle, and 16 particles
@@ -341,7 +344,7 @@ int hist_split(uint32_t ntiles) { return ntiles <= 37 ? 8 : ntiles <= 148 ? 4 : 
 void launch_kick_drift_bbox(const StepBufs& b, int kick, int pending, cudaStream_t st) {
   const int split = stream_split(b.ntiles);
   k_kick_drift_bbox<<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.sys, b.pos, b.vel, b.acc, kick, pending,
-                                                               b.bbox_enc, split);
+                                                               b.bbox_enc, b.slots, split);
 }
 
 uint32_t small_sort_max() { return kTile; }
@@ -371,15 +374,10 @@ void launch_kick_half(const StepBufs& b, cudaStream_t st) {
 
 void launch_morton_hist(const StepBufs& b, uint32_t* lanes_out, cudaStream_t st) {
   const int split = hist_split(b.ntiles);
-  if (b.key64)
-    k_morton_hist<true, kRadixBits><<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.pos, b.bbox_enc, b.sys, b.bounds,
-                                                                        b.codes, nullptr, b.hist, split);
-  else if (b.radix_bits == kRadixBitsWide)
-    k_morton_hist<false, kRadixBitsWide><<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.pos, b.bbox_enc, b.sys,
-                                                                             b.bounds, b.codes, lanes_out, b.hist, split);
-  else
-    k_morton_hist<false, kRadixBits><<<b.ntiles * split, kTileThreads, 0, st>>>(b.tiles, b.pos, b.bbox_enc, b.sys, b.bounds,
-                                                                         b.codes, lanes_out, b.hist, split);
+  auto kern = b.key64 ? k_morton_hist<true, kRadixBits>
+              : b.radix_bits == kRadixBitsWide ? k_morton_hist<false, kRadixBitsWide> : k_morton_hist<false, kRadixBits>;
+  launch_after(b.ntiles, kern, b.ntiles * split, kTileThreads, 0, st, b.tiles, b.pos, b.bbox_enc, b.sys, b.bounds, b.codes,
+               b.key64 ? nullptr : lanes_out, b.hist, split);
 }
 
 }  // namespace gx
