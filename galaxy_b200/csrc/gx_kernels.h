@@ -67,7 +67,7 @@ struct StepBufs {
 
 // CTAs of kWalkThreads threads per SM that the FP32 walk's shared memory allows, with
 // monopoles and with quadrupoles.
-constexpr int kWalkCtas = 4, kWalkCtasQuad = 3;
+constexpr int kWalkCtas = 4, kWalkCtasQuad = 4;
 
 // Launches kern after the kernel before it on st, to be scheduled as that one drains; kern
 // begins with step_kernel_begin. That takes about 1 us off the gap to the kernel before
@@ -113,9 +113,12 @@ void launch_morton_hist(const StepBufs& b, uint32_t* lanes_out, cudaStream_t st)
 void launch_sort(const StepBufs& b, cudaStream_t st);
 // the four passes on explicit buffers: keys_in -> (keys_out, vals_out), values start as
 // the identity; keys_tmp/vals_tmp hold passes 0 and 2
+// key_bits: the keys' width, which sets the number of passes; an odd number needs a third
+// key buffer keys_tmp2 (keys_in itself may serve: only the first pass reads it).
 void launch_sort_passes(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_out, uint32_t* keys_tmp,
                         uint32_t* vals_tmp, const TileDesc* tiles, const SysDesc* sys, const uint32_t* hist,
-                        uint32_t* status, uint32_t* counters, uint32_t ntiles, DevCtl* ctl, cudaStream_t st);
+                        uint32_t* status, uint32_t* counters, uint32_t ntiles, DevCtl* ctl, cudaStream_t st,
+                        int key_bits = 32, uint32_t* keys_tmp2 = nullptr);
 // per-system digit histograms of b.codes (when codes come from the host)
 void launch_code_hist(const StepBufs& b, cudaStream_t st);
 // gx_build.cu: gather leaves + bottom-up Karras build and aggregation

@@ -279,9 +279,12 @@ __global__ void __launch_bounds__(kTileThreads) k_code_hist(const TileDesc* __re
 
 void launch_sort_passes(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_out, uint32_t* keys_tmp,
                         uint32_t* vals_tmp, const TileDesc* tiles, const SysDesc* sys, const uint32_t* hist,
-                        uint32_t* status, uint32_t* counters, uint32_t ntiles, DevCtl* ctl, cudaStream_t st) {
-  run_passes<uint32_t, kRadixBits>(kRadixPasses, keys_in, keys_out, vals_out, keys_tmp, nullptr, vals_tmp, tiles, sys,
-                                   hist, status, counters, ntiles, ctl, st);
+                        uint32_t* status, uint32_t* counters, uint32_t ntiles, DevCtl* ctl, cudaStream_t st,
+                        int key_bits, uint32_t* keys_tmp2) {
+  int passes = (key_bits + kRadixBits - 1) / kRadixBits;
+  if (passes < 1 || passes > kRadixPasses || (passes % 2 != 0 && !keys_tmp2)) passes = kRadixPasses;
+  run_passes<uint32_t, kRadixBits>(passes, keys_in, keys_out, vals_out, keys_tmp, keys_tmp2, vals_tmp, tiles, sys, hist,
+                                   status, counters, ntiles, ctl, st);
 }
 
 void launch_code_hist(const StepBufs& b, cudaStream_t st) {
