@@ -200,34 +200,15 @@ __device__ __forceinline__ void write_rest(const StepBufs& b, uint32_t gi, const
   }
 }
 
-// Fold the held node with its sibling into their parent (fold_agg's order: left, then
-// right); the parent becomes the held node. LEFT: the held node is the left child. The
-// side is a template argument so that every operand is named directly (a run-time
-// choice between the two aggregates would take their addresses and move them to the
-// local-memory stack).
-template <bool QUAD, bool LEFT>
-__device__ __forceinline__ void combine_side(Climb& c, const AggR& sib, const double sq[6], uint32_t sib_u,
-                                             uint32_t sib_far, uint32_t n_total, double theta, double inv_theta,
-                                             double tiny2) {
-  const AggR& CL = LEFT ? c.cur : sib;
-  const AggR& CR = LEFT ? sib : c.cur;
+// Fold children CL and CR (quadrupoles qL, qR) into c.cur (c.q), in fold_agg's order: left,
+// then right.
+template <bool QUAD>
+__device__ __forceinline__ void fold_pair(Climb& c, const AggR& CL, const AggR& CR, const double qL[6],
+                                          const double qR[6]) {
   AggR par;
   fold(CL, CR, par);
-  if (LEFT) {
-    c.lc = c.u;
-    c.rc = sib_u;
-    c.r = sib_far;
-  } else {
-    c.lc = sib_u;
-    c.rc = c.u;
-    c.l = sib_far;
-  }
-  c.pl = child_record(CL, c.lc < n_total, theta, inv_theta, tiny2);
-  c.pr = child_record(CR, c.rc < n_total, theta, inv_theta, tiny2);
   if (QUAD) {
     // Q_parent = shift(Q_left) + shift(Q_right), left first (oracle order).
-    const double* qL = LEFT ? c.q : sq;
-    const double* qR = LEFT ? sq : c.q;
     double dl[3], dr[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -243,14 +224,38 @@ __device__ __forceinline__ void combine_side(Climb& c, const AggR& sib, const do
   c.cur = par;
 }
 
+// Fold the held node with its sibling into their parent, which becomes the held node. The
+// sides are chosen value by value: lanes of both sides fold together (a branch on the side
+// would run the fold and both records twice in nearly every warp).
 template <bool QUAD>
 __device__ __forceinline__ void combine(Climb& c, const AggR& sib, const double sq[6], bool is_left, uint32_t sib_u,
                                         uint32_t sib_far, uint32_t n_total, double theta, double inv_theta,
                                         double tiny2) {
-  if (is_left)
-    combine_side<QUAD, true>(c, sib, sq, sib_u, sib_far, n_total, theta, inv_theta, tiny2);
-  else
-    combine_side<QUAD, false>(c, sib, sq, sib_u, sib_far, n_total, theta, inv_theta, tiny2);
+  AggR CL, CR;
+  double qL[6], qR[6];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    CL.mn[k] = is_left ? c.cur.mn[k] : sib.mn[k];
+    CR.mn[k] = is_left ? sib.mn[k] : c.cur.mn[k];
+    CL.mx[k] = is_left ? c.cur.mx[k] : sib.mx[k];
+    CR.mx[k] = is_left ? sib.mx[k] : c.cur.mx[k];
+    CL.com[k] = is_left ? c.cur.com[k] : sib.com[k];
+    CR.com[k] = is_left ? sib.com[k] : c.cur.com[k];
+  }
+  CL.m = is_left ? c.cur.m : sib.m;
+  CR.m = is_left ? sib.m : c.cur.m;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    qL[k] = is_left ? c.q[k] : sq[k];
+    qR[k] = is_left ? sq[k] : c.q[k];
+  }
+  c.lc = is_left ? c.u : sib_u;
+  c.rc = is_left ? sib_u : c.u;
+  c.l = is_left ? c.l : sib_far;
+  c.r = is_left ? sib_far : c.r;
+  c.pl = child_record(CL, c.lc < n_total, theta, inv_theta, tiny2);
+  c.pr = child_record(CR, c.rc < n_total, theta, inv_theta, tiny2);
+  fold_pair<QUAD>(c, CL, CR, qL, qR);
 }
 
 constexpr int kDeltaMax = 0x7fffffff;  // "no pair": past the end of a block's leaves
@@ -437,27 +442,11 @@ __global__ void __launch_bounds__(kBuildLeaves, (QUAD ? 2 : 3) * (256 / kBuildLe
         const uint32_t gi = off + (root ? 0u : (is_left ? c.r : c.l));
         const uint32_t li = gi - first;  // inside the block: first <= gi < first + m
         c.u = n_total + gi;
-        S.kids[li] = make_uint2(c.lc, c.rc);
-        if (c.lc < n_total)
-          S.par_leaf[c.lc - first] = c.u;
-        else
-          S.par_int[c.lc - n_total - first] = c.u;
-        if (c.rc < n_total)
-          S.par_leaf[c.rc - first] = c.u;
-        else
-          S.par_int[c.rc - n_total - first] = c.u;
         S.inr[li] = c.cur;
         if (QUAD) {
 #pragma unroll
           for (int a = 0; a < 6; ++a) S.q[6 * li + a] = c.q[a];
         }
-        float4* pp = S.pairs + 5 * li;
-        pp[0] = make_float4(c.pl.hx, c.pr.hx, c.pl.hy, c.pr.hy);
-        pp[1] = make_float4(c.pl.hz, c.pr.hz, c.pl.m, c.pr.m);
-        pp[2] = make_float4(c.pl.lx, c.pr.lx, c.pl.ly, c.pr.ly);
-        pp[3] = make_float4(c.pl.lz, c.pr.lz, c.pl.take, c.pr.take);
-        pp[4] = make_float4(c.pl.open, c.pr.open, __uint_as_float(child_code(c.lc, n_total)),
-                            __uint_as_float(child_code(c.rc, n_total)));
         if (root) {
           S.par_int[li] = kNoParent;
           go = false;
@@ -506,49 +495,68 @@ __global__ void __launch_bounds__(kBuildLeaves, (QUAD ? 2 : 3) * (256 / kBuildLe
     if (fold) S.work[base + __popc(fb & ((1u << lane) - 1u))] = item;
     __syncthreads();  // the round's folds are listed (and every thread has read the counts)
     if (total == 0) break;
-    // (B) fold item tid: the node that arrived second and its sibling, both from shared memory
-    if (tid < total) {
-      const uint2 w = S.work[tid];
+    // (B) the round's folds (at most half as many as the block has leaves): the first half of
+    // the block folds item tid, the second half computes the same item's walk records and
+    // links, beside it instead of after it. Left and right child are taken from shared memory
+    // by index, so no warp runs both sides. (One thread for both and a branch on the side:
+    // the stage 384 us at 2^20 particles, 97 us at 16,384; this way 320 and 85 us.)
+    const bool records = tid >= kBuildLeaves / 2;
+    const int job = records ? tid - kBuildLeaves / 2 : tid;
+    if (job < total) {
+      const uint2 w = S.work[job];
       const uint32_t xi = w.x & 255u, si = w.y & 255u;
       const bool x_leaf = (w.x & 256u) != 0, sib_leaf = (w.y & 256u) != 0;
       const bool is_left = ((w.x >> 25) & 1u) != 0;
-      c.l = clo + ((w.x >> 9) & 255u);
-      c.r = clo + ((w.x >> 17) & 255u);
-      c.u = x_leaf ? first + xi : n_total + first + xi;
-      const uint32_t sib_u = sib_leaf ? first + si : n_total + first + si;
+      const uint32_t xl = clo + ((w.x >> 9) & 255u), xr = clo + ((w.x >> 17) & 255u);
       const uint32_t sib_far = clo + ((w.y >> 9) & 255u);
-      AggR sib;
-      double sq[6] = {0, 0, 0, 0, 0, 0};
-      if (x_leaf) {
-        const double4 lf = S.leaf[xi];
-        c.cur.com[0] = c.cur.mn[0] = c.cur.mx[0] = lf.x;
-        c.cur.com[1] = c.cur.mn[1] = c.cur.mx[1] = lf.y;
-        c.cur.com[2] = c.cur.mn[2] = c.cur.mx[2] = lf.z;
-        c.cur.m = lf.w;
-#pragma unroll
-        for (int a = 0; a < 6; ++a) c.q[a] = 0.0;
-      } else {
-        c.cur = S.inr[xi];
+      const uint32_t iL = is_left ? xi : si, iR = is_left ? si : xi;
+      const bool leafL = is_left ? x_leaf : sib_leaf, leafR = is_left ? sib_leaf : x_leaf;
+      auto load = [&](uint32_t i, bool leaf, AggR& a) {
+        if (leaf) {
+          const double4 lf = S.leaf[i];
+          a.com[0] = a.mn[0] = a.mx[0] = lf.x;
+          a.com[1] = a.mn[1] = a.mx[1] = lf.y;
+          a.com[2] = a.mn[2] = a.mx[2] = lf.z;
+          a.m = lf.w;
+        } else {
+          a = S.inr[i];
+        }
+      };
+      AggR CL, CR;
+      load(iL, leafL, CL);
+      load(iR, leafR, CR);
+      c.l = is_left ? xl : sib_far;
+      c.r = is_left ? sib_far : xr;
+      if (!records) {
+        double qL[6], qR[6];
         if (QUAD) {
 #pragma unroll
-          for (int a = 0; a < 6; ++a) c.q[a] = S.q[6 * xi + a];
+          for (int a = 0; a < 6; ++a) {
+            qL[a] = leafL ? 0.0 : S.q[6 * iL + a];
+            qR[a] = leafR ? 0.0 : S.q[6 * iR + a];
+          }
         }
-      }
-      if (sib_leaf) {
-        const double4 lf = S.leaf[si];
-        sib.com[0] = sib.mn[0] = sib.mx[0] = lf.x;
-        sib.com[1] = sib.mn[1] = sib.mx[1] = lf.y;
-        sib.com[2] = sib.mn[2] = sib.mx[2] = lf.z;
-        sib.m = lf.w;
+        fold_pair<QUAD>(c, CL, CR, qL, qR);
+        held = true;
       } else {
-        sib = S.inr[si];
-        if (QUAD) {
-#pragma unroll
-          for (int a = 0; a < 6; ++a) sq[a] = S.q[6 * si + a];
-        }
+        const int d_lo = S.d[c.l - clo], d_hi = S.d[c.r - clo + 1];
+        const bool root = d_lo < 0 && d_hi < 0;
+        const uint32_t gi = off + (root ? 0u : (d_hi > d_lo ? c.r : c.l));
+        const uint32_t li = gi - first, u = n_total + gi;
+        const uint32_t lc = leafL ? first + iL : n_total + first + iL, rc = leafR ? first + iR : n_total + first + iR;
+        S.kids[li] = make_uint2(lc, rc);
+        (leafL ? S.par_leaf : S.par_int)[iL] = u;
+        (leafR ? S.par_leaf : S.par_int)[iR] = u;
+        const ChildRec pl = child_record(CL, leafL, theta, inv_theta, tiny2);
+        const ChildRec pr = child_record(CR, leafR, theta, inv_theta, tiny2);
+        float4* pp = S.pairs + 5 * li;
+        pp[0] = make_float4(pl.hx, pr.hx, pl.hy, pr.hy);
+        pp[1] = make_float4(pl.hz, pr.hz, pl.m, pr.m);
+        pp[2] = make_float4(pl.lx, pr.lx, pl.ly, pr.ly);
+        pp[3] = make_float4(pl.lz, pr.lz, pl.take, pr.take);
+        pp[4] = make_float4(pl.open, pr.open, __uint_as_float(child_code(lc, n_total)),
+                            __uint_as_float(child_code(rc, n_total)));
       }
-      combine<QUAD>(c, sib, sq, is_left, sib_u, sib_far, n_total, theta, inv_theta, tiny2);
-      held = true;
     }
     internal = true;
   }
