@@ -276,10 +276,12 @@ void tuned_store(int device, const gx_options& opt, int batched, size_t n, const
 
 // Targets a warp of the FP32 walk when nothing is tuned: narrow groups for small systems,
 // whose walk is the latency of few warps (more warps, tighter group boxes), 32 targets
-// for large ones. Measured at 8 / 16 / 32 targets (walk, us): Plummer 16,384 135 / 158 /
-// 217; disk 40,000 162 / 135 / 158; Plummer 100,000 776 / 588 / 580; disk 200,003 1272 /
-// 969 / 926; collisions of 262,144 2435 / 1796 / 1669 and 1,048,576 - / 5423 / 4714.
-uint32_t default_walk_group(size_t n) { return n < (size_t{1} << 15) ? 8u : n < (size_t{1} << 17) ? 16u : 32u; }
+// for large ones. 16 targets would be 15% faster from 2^15 on and 32 5-10% from 2^17 on
+// (walk at 8 / 16 / 32 targets, us: disk 40,000 162 / 135 / 158; disk 200,003 1272 / 969 /
+// 926; collision 262,144 2435 / 1796 / 1669), but the grouping sets which terms are rounded
+// relative to which box, and so the last bits of every default result: it stays, and
+// gx_autotune finds the faster one.
+uint32_t default_walk_group(size_t n) { return n < (size_t{1} << 16) ? 8u : n < (size_t{1} << 19) ? 16u : 32u; }
 
 uint32_t system_radix_bits(int device, const gx_options& opt, size_t n) {
   if (opt.flags & GX_FLAG_MORTON63) return kRadixBits;

@@ -331,18 +331,18 @@ constexpr int kWalkStack = 384;  // stack entries
 constexpr int kWalkDeep = kWalkStack - kMaxDepth - 36;  // stack entries the wide rounds may fill
 constexpr int kWalkList = 96;    // entries per list: at most 31 left after an evaluation + 64 a round
 constexpr int kWalkFlush = 32;   // a list is evaluated once it holds this many entries
-// Undecided and near entries together: at most 31 of each are left over and a round adds at
-// most 64; a batch of undecided entries moves at most its own number to the near list.
+// Undecided and near entries together: at most 31 of each are left over, a round adds at most
+// 64 undecided ones and a batch of those moves at most its own number to the near list.
 constexpr int kWalkPool = 128;
 static_assert(31 + 31 + 64 <= kWalkPool, "undecided and near entries");
-// An entry is evaluated relative to the centre of the targets' box when the box's far
-// corner is at most sqrt(kNearRatio) times as far from it as any target that takes it: the
-// rounding of the two relative coordinates is then a few 2^-24 of their difference. Nearer
-// entries (the warp's own leaves and their neighbours, a few percent) keep float-float
-// coordinates, whose difference is exact to 2^-24 of itself. Measured on the collision of
-// 2^20 (walk, relative error against 64 bits): no near list 4.58 ms 3.4e-8 (a disk of
-// 200,003: 9.2e-8, where 3.9e-8 is reached with one), ratio 1024 4.88 ms 3.25e-8, 256 4.91
-// ms 3.23e-8, 64 4.93 ms 3.22e-8, 16 5.12 ms 3.19e-8, 4 5.56 ms 3.14e-8.
+// What some targets of an undecided entry take is evaluated relative to the centre of the
+// targets' box when the box's far corner is at most sqrt(kNearRatio) times as far from the
+// entry as any target that takes it: the rounding of the two relative coordinates is then
+// a few 2^-24 of their difference. Nearer entries keep float-float coordinates, whose
+// difference is exact to 2^-24 of itself. (With every undecided entry relative, the error
+// against 64-bit sums grew: a disk of 200,003 1.1e-7 -> 1.3e-7, an active subset of a disk
+// 3.7e-7 -> 5.0e-7. Ratios of 4, 16, 64, 256 and 1024 cost 5.56, 5.12, 4.93, 4.91 and 4.88
+// ms on the collision of 2^20 when the group-accepted entries were held to them too.)
 constexpr float kNearRatio = 256.f;
 constexpr uint32_t kNearCode = 0x40000000u;  // flag of an undecided entry's code (indices are below 2^30)
 constexpr float kGroupHi = 1.0f + 0x1p-20f;
@@ -373,10 +373,10 @@ __device__ __forceinline__ void put2(float4* a, int e, float v0, float v1) {
 //        two entries share each float4: entry e is half (e & 1) of float4 e >> 1;
 //   undecided list: children some targets take and others open (or that need the FP64
 //        re-decision), one field an array: a lane decides one entry for every target;
-//   near list: children to be taken like the dense ones, but so close to the targets,
-//        for the size of the targets' box, that coordinates relative to its centre would
-//        lose bits (kNearRatio): they keep float-float coordinates. It grows down from the
-//        end of the undecided list's arrays;
+//   near list: once undecided children that some targets take, so close to the targets, for
+//        the size of the targets' box, that coordinates relative to its centre would lose
+//        bits (kNearRatio): they keep float-float coordinates. It grows down from the end
+//        of the undecided list's arrays;
 //   targets: the float-float coordinates of the warp's targets, negated, two a float4, so
 //        that one broadcast load serves the packed instructions of two targets.
 struct WarpLists {
@@ -495,8 +495,7 @@ __device__ __forceinline__ void quad2(float2 dx, float2 dy, float2 dz, float2 in
 // re-decision in the band, the inside test for theta >= kInsideTheta): the masks of the
 // targets that take and that open the entry build up in the lane's registers. (Deciding
 // an entry for a target a lane costs six shared loads, two ballots and a vote an entry;
-// this way none: the collision of 2^20 at theta 0.5, 6.0 -> 4.7 ms, and its error against
-// 64-bit sums 4.1e-8 -> 3.2e-8.) An entry
+// this way none: the collision of 2^20 at theta 0.5, 6.0 -> 4.5 ms.) An entry
 // some targets open goes back on the stack for them, one some targets take goes on the
 // dense list for them. The dense list is evaluated a target a lane (the R lanes of a
 // target take turns over its entries), four entries a lane-iteration with packed FP32 and
@@ -693,13 +692,9 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
         const bool opnL = act && !accL && dmax2.x * kGroupHi < r4.x;
         const bool opnR = act && !accR && dmax2.y * kGroupHi < r4.y;
         const bool undL = act && !accL && !opnL, undR = act && !accR && !opnR;
-        // too near for box-relative coordinates: what is taken is farther than dmin, and
-        // than the take threshold
+        // undecided and too near for box-relative coordinates: what is taken is farther than
+        // dmin, and than the take threshold
         const bool nearL = dmax2.x > kNearRatio * fmaxf(dmin2.x, r3.z), nearR = dmax2.y > kNearRatio * fmaxf(dmin2.y, r3.w);
-        const bool nrL = accL && nearL, nrR = accR && nearR;
-        const uint32_t bNL = __ballot_sync(0xffffffffu, nrL), bNR = __ballot_sync(0xffffffffu, nrR);
-        accL = accL && !nearL;
-        accR = accR && !nearR;
         const uint32_t bAL = __ballot_sync(0xffffffffu, accL), bAR = __ballot_sync(0xffffffffu, accR);
         const uint32_t bUL = __ballot_sync(0xffffffffu, undL), bUR = __ballot_sync(0xffffffffu, undR);
         const uint32_t bOL = __ballot_sync(0xffffffffu, opnL), bOR = __ballot_sync(0xffffffffu, opnR);
@@ -729,14 +724,11 @@ __global__ void __launch_bounds__(kWalkThreads, GX_WALK_MINB) k_walk_f32(StepBuf
           if (accR) put_dense(eAR, rx.y, ry.y, rz.y, r1.w, M, cR);
         }
         dl += __popc(bAL) + __popc(bAR);
-        if (undL || nrL)
-          put_und(undL ? eUL : kWalkPool - 1 - (nl + __popc(bNL & lt)), chx.x, chy.x, chz.x, r1.z, clx.x, cly.x, clz.x,
-                  r3.z, r4.x, cL | (undL && nearL ? kNearCode : 0u), M);
-        if (undR || nrR)
-          put_und(undR ? eUR : kWalkPool - 1 - (nl + __popc(bNL) + __popc(bNR & lt)), chx.y, chy.y, chz.y, r1.w, clx.y,
-                  cly.y, clz.y, r3.w, r4.y, cR | (undR && nearR ? kNearCode : 0u), M);
+        if (undL)
+          put_und(eUL, chx.x, chy.x, chz.x, r1.z, clx.x, cly.x, clz.x, r3.z, r4.x, cL | (nearL ? kNearCode : 0u), M);
+        if (undR)
+          put_und(eUR, chx.y, chy.y, chz.y, r1.w, clx.y, cly.y, clz.y, r3.w, r4.y, cR | (nearR ? kNearCode : 0u), M);
         ul += __popc(bUL) + __popc(bUR);
-        nl += __popc(bNL) + __popc(bNR);
         const int npush = __popc(bOL) + __popc(bOR);
         if (sp + npush > kWalkStack) {
           bad = true;
