@@ -678,9 +678,9 @@ def run_precision(args):
 
 
 # Kernels a gas-mode step adds to the 9 of the gravity step: gather, scalars, 3 grids
-# (keys, histogram, 4 sort passes, fill, mixed flags), seeds, density cell, density, h_max,
-# hydro cell, pack, hydro, scatter.
-SPH_LAUNCHES_PER_STEP = 2 + 3 * 8 + 8
+# (keys, histogram, 3 sort passes, fill, mixed flags), seeds, density cell, density, h_max,
+# hydro cell, pack, reach, hydro, scatter.
+SPH_LAUNCHES_PER_STEP = 2 + 3 * 7 + 9
 
 
 def sph_roofline(n_gas: int, stage: dict, peaks: dict) -> dict:
