@@ -677,10 +677,12 @@ def run_precision(args):
         dist.destroy_process_group()
 
 
-# Kernels a gas-mode step adds to the 9 of the gravity step: gather, scalars, 3 grids
-# (keys, histogram, 3 sort passes, fill, mixed flags), seeds, density cell, density, h_max,
-# hydro cell, pack, reach, hydro, scatter.
-SPH_LAUNCHES_PER_STEP = 2 + 3 * 7 + 9
+# Kernels a gas-mode step adds to the 9 of the gravity step when bucket numbers take four sort
+# passes: gather, scalars, 3 grids (keys, histogram, 4 sort passes, fill, mixed flags), seeds,
+# density cell, density, h_max, hydro cell, pack, hydro, scatter. Up to 2^24 buckets three
+# passes sort them (3 fewer), and the reach kernel adds one.
+SPH_LAUNCHES_PER_STEP = 2 + 3 * 8 + 8
+SPH_LAUNCHES_NOW = SPH_LAUNCHES_PER_STEP - 3 + 1
 
 
 def sph_roofline(n_gas: int, stage: dict, peaks: dict) -> dict:
@@ -801,7 +803,7 @@ def run_sph(args):
                            "l2": f"working set ~{900 * n / 1e6:.0f} MB > 126 MB L2 (no flush needed)",
                            "walk_launch": {k: tune[k] for k in ("walk_block", "walk_ctas_per_sm", "walk_group")}},
                 "gas_particle_steps_per_s": ng * ws * args.steps / (ms_max / 1e3),
-                "e2e": e2e, "gpu_launches": (9 + SPH_LAUNCHES_PER_STEP) * args.steps, "cpu_baseline": cpu,
+                "e2e": e2e, "gpu_launches": (9 + SPH_LAUNCHES_NOW) * args.steps, "cpu_baseline": cpu,
                 "clocks": clk, "stage_ms": stage, "sph_share_of_step": gas_frac, "min_stable_dt_c0.25": cfl,
                 "roofline": sph_roofline(ng, stage, peaks)}
         print(json.dumps(line), flush=True)
