@@ -173,7 +173,11 @@ __device__ __forceinline__ double warp_max(double v) {
 // Every gas particle whose cell lies in the query box of centre c and half-width R,
 // each exactly once: f(ok, slot) is called by all 32 lanes together (ok false for
 // padding lanes and for bucket entries of another cell; a bucket that holds one cell is
-// checked once, by its first entry). A box wider than the limits visits every slot instead.
+// checked once, by its first entry). A box wider than the limits, or of more cells than
+// there are particles, visits every slot instead: a cell costs at least what a slot does.
+// (Force calls with a cold density, us, by the limits alone / at more than 4 / more than 1
+// cell a particle: 300 particles, one far away, 3053 / 352 / 357; 3,000, 15 far away, 4608 /
+// 1339 / 1254; 9,000 of a Plummer sphere 13448 / 13515 / 6484; cubes and disks the same.)
 // keep(bucket, x, y, z, cell): whether a non-empty cell can hold a particle that f wants
 // (only asked of cells inside the limits).
 template <class P, class F>
@@ -186,7 +190,7 @@ __device__ __forceinline__ void visit_box_if(const GridDev& g, double cx, double
   const int lz = cell_coord(cz - R, cell), hz = cell_coord(cz + R, cell);
   const long long nx = static_cast<long long>(hx) - lx + 1, ny = static_cast<long long>(hy) - ly + 1,
                   nz = static_cast<long long>(hz) - lz + 1;
-  if (nx > kBoxAxisMax || ny > kBoxAxisMax || nz > kBoxAxisMax || nx * ny * nz > kBoxCellsMax) {
+  if (nx > kBoxAxisMax || ny > kBoxAxisMax || nz > kBoxAxisMax || nx * ny * nz > min(kBoxCellsMax, g.n)) {
     for (uint32_t s0 = 0; s0 < g.n; s0 += 32) f(s0 + lane < g.n, s0 + lane);
     return;
   }

@@ -42,3 +42,26 @@ def test_h_matches_oracle(oracle, kind, n, n_ngb):
             ref_rho2, ref_h2 = ref_rho, ref_h
         assert np.allclose(h, ref_h2, rtol=1e-12, atol=0.0)
         assert np.allclose(rho, ref_rho2, rtol=1e-11, atol=0.0)
+
+
+def test_far_outliers_cost_about_as_much():
+    # Boxes that span thousands of empty cells must not be gone through cell by cell when
+    # there are fewer particles than cells: the call with one particle far away took 8.5
+    # times as long as without it, and takes 1.0 times.
+    import time
+
+    rng = np.random.default_rng(5)
+    pos, mass = rng.random((300, 3)), np.full(300, 1.0 / 300)
+    far = pos.copy()
+    far[0] = far[0] * 40.0 - 20.0
+    s = gb.GpuGravitySph(1.0, 0.01, 0.5)
+
+    def best(p):
+        t = []
+        for _ in range(30):
+            t0 = time.perf_counter()
+            s.density(p, mass)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    assert best(far) <= 4.0 * best(pos)
