@@ -732,7 +732,8 @@ __global__ void __launch_bounds__(kFlat) k_sph_reach(GridDev g, const SphScalars
   for (uint32_t s = blockIdx.x * kFlat + threadIdx.x; s < g.n; s += gridDim.x * kFlat) {
     const int4 c = g.sc[s];
     uint32_t m = 0;
-    if (max(max(abs(c.x), abs(c.y)), abs(c.z)) > (1 << 30)) {
+    auto edge = [](int v) { return v > (1 << 30) || v < -(1 << 30); };
+    if (edge(c.x) || edge(c.y) || edge(c.z)) {  // clamped (or nearly): v +- 2 might not be an int
       m = top;
     } else {
       for (int z = -2; z <= 2; ++z)
