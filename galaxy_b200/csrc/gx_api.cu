@@ -329,6 +329,7 @@ struct gx_handle {
   cudaEvent_t ev[8] = {};  // stage boundaries; [5] gx_step_many_timed, [6] end of SPH, [7] end of its density
   cudaEvent_t chunk_ev[8] = {};  // gx_kdk_step_host: acceleration chunks copied back
   DevCtl* ctl_host = nullptr;     // pinned copy of the device error word
+  char* small_out = nullptr;      // behind it, kSmallOut bytes for copy_out
   std::string err;
   Arena ar;
   // current layout
@@ -369,6 +370,9 @@ struct gx_handle {
 };
 
 namespace {
+
+constexpr size_t kCtlRoom = 256;  // ctl_host's part of the handle's pinned memory
+static_assert(sizeof(DevCtl) <= kCtlRoom, "room of the error word");
 
 int fail(gx_handle* h, int code, const std::string& msg) {
   if (h) h->err = msg;
@@ -502,7 +506,7 @@ int finish(gx_handle* h, bool timed, const HostPiece* outs = nullptr, int n_outs
   if (h->ar.b.ctl)
     GX_CK(h, cudaMemcpyAsync(h->ctl_host, h->ar.b.ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, h->stream));
   if (n_outs)
-    GX_CK(h, copy_out(h->device, h->stream, outs, n_outs));
+    GX_CK(h, copy_out(h->device, h->stream, outs, n_outs, h->small_out));
   else
     GX_CK(h, cudaStreamSynchronize(h->stream));
   GX_CK(h, cudaGetLastError());
@@ -617,7 +621,8 @@ int gx_create(double g, double softening, double theta, const gx_options* opt, g
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
   for (int i = 0; i < 8 && e == cudaSuccess; ++i) e = cudaEventCreate(&h->ev[i]);
   for (int i = 0; i < 8 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&h->chunk_ev[i], cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaHostAlloc(&h->ctl_host, sizeof(DevCtl), cudaHostAllocDefault);
+  if (e == cudaSuccess) e = cudaHostAlloc(&h->ctl_host, kCtlRoom + kSmallOut, cudaHostAllocDefault);
+  h->small_out = reinterpret_cast<char*>(h->ctl_host) + kCtlRoom;
   if (e != cudaSuccess) {
     set_global_err(std::string("stream/event creation failed: ") + cudaGetErrorString(e));
     delete h;
