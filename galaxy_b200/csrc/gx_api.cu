@@ -888,6 +888,20 @@ int gx_synchronize(gx_handle* h) {
   return finish(h, stats_on(h));  // stage times of the last step when they are on
 }
 
+namespace {
+// The sum of the potential's partials (Neumaier's compensated sum; one that is not finite
+// stays as it is).
+double potential_total(const std::vector<double>& part) {
+  double s = 0.0, c = 0.0;
+  for (double v : part) {
+    const double t = s + v;
+    if (std::isfinite(t)) c += std::fabs(s) >= std::fabs(v) ? (s - t) + v : (v - t) + s;
+    s = t;
+  }
+  return s + c;
+}
+}  // namespace
+
 int gx_potential_energy(gx_handle* h, size_t n, const double* pos, const double* mass, double* out) {
   if (!h || !out) return GX_ERR_INVALID_ARG;
   *out = 0.0;
@@ -905,9 +919,7 @@ int gx_potential_energy(gx_handle* h, size_t n, const double* pos, const double*
   std::vector<double> part(np);
   GX_CK(h, cudaMemcpyAsync(part.data(), h->ar.diag_partial, np * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   GX_CK(h, cudaStreamSynchronize(h->stream));
-  double u = 0.0;
-  for (double v : part) u += v;
-  *out = u;
+  *out = potential_total(part);
   return GX_OK;
 }
 
@@ -1227,7 +1239,7 @@ int gx_diagnostics(gx_handle* h, int with_potential, double* out) {
     std::vector<double> pp(np);
     GX_CK(h, cudaMemcpyAsync(pp.data(), h->ar.diag_partial, np * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     GX_CK(h, cudaStreamSynchronize(h->stream));
-    for (double v : pp) out[1] += v;
+    out[1] = potential_total(pp);
   }
   return finish(h, false);
 }

@@ -69,18 +69,6 @@ __global__ void __launch_bounds__(kDiagThreads) k_direct_sum_f64(uint32_t n, con
     for (int c = 0; c < 3; ++c) acc[3 * (size_t)t + c] = a[c] * g;
 }
 
-// 1 / sqrt(x) to double precision: the hardware's approximation (about 2^-22.5 relative)
-// and one step of Householder's third-order iteration, y (1 + e/2 + 3 e^2 / 8) with
-// e = 1 - x y^2 (its error, 5/16 e^3, is below 2^-66). Zero, subnormal, infinite and NaN
-// arguments take the library function.
-__device__ __forceinline__ double inv_sqrt(double x) {
-  if (static_cast<uint32_t>(__double2hiint(x) - 0x00100000) >= 0x7fe00000u) return rsqrt(x);
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(e * y, fma(e, 0.375, 0.5), y);
-}
-
 constexpr int kPotThreads = 128;
 constexpr int kPotTile = 256;  // rows and columns of a unit: two rows a thread
 
@@ -88,9 +76,11 @@ constexpr int kPotTile = 256;  // rows and columns of a unit: two rows a thread
 // rows by kPotTile columns on and above the diagonal (half of the double sum), taken by
 // the blocks in turn, so that a few thousand units of equal work keep every SM busy
 // whatever N is. FP64-bound: 12 FP64 operations a pair. partial[b] = block b's sum, in a
-// fixed order. (A thread a row over all columns, with half the pairs counted twice, one
-// block a 256 rows and the library's rsqrt: N = 65,537 in 7.3 ms; this way 2.3 ms, 21 of the
-// 37 FP64 TFLOP/s.)
+// fixed order; the host adds the up to 2,368 partials with compensation (potential_total).
+// (A thread a row over all columns, half the pairs counted twice, one block a 256 rows: a
+// call at 100 / 300 / 1,000 / 65,537 / 131,072 particles in 42 / 70 / 143 / 7,430 / 25,400 us; this
+// way 41 / 62 / 81 / 2,250 / 8,340. Mean error against 80-bit sums over 64 to 20,011
+// particles: 1.2e-16 and 5.7e-17; 2.8e-16 with a plain sum of the partials.)
 __global__ void __launch_bounds__(kPotThreads) k_potential_f64(uint32_t n, const double* __restrict__ pos,
                                                                const double* __restrict__ mass, double g, double eps2,
                                                                double* __restrict__ partial) {
@@ -99,18 +89,21 @@ __global__ void __launch_bounds__(kPotThreads) k_potential_f64(uint32_t n, const
   const int tid = threadIdx.x;
   const unsigned long long tiles = (n + kPotTile - 1u) / kPotTile, units = tiles * (tiles + 1ull) / 2ull;
   double total = 0.0;
+  // The thread's rows of a tile. The second ones go to the warps in reverse, so that on the
+  // diagonal, where later rows have fewer columns, every warp has as much to do.
+  const uint32_t row[2] = {static_cast<uint32_t>(tid), static_cast<uint32_t>(kPotThreads + (tid ^ (kPotThreads - 32)))};
   for (unsigned long long u = blockIdx.x; u < units; u += gridDim.x) {
     // unit u is (row tile I, column tile J) with u = J (J + 1) / 2 + I, I <= J
     unsigned long long J = static_cast<unsigned long long>((sqrt(8.0 * static_cast<double>(u) + 1.0) - 1.0) * 0.5);
     while (J * (J + 1ull) / 2ull > u) --J;
     while ((J + 1ull) * (J + 2ull) / 2ull <= u) ++J;
     const unsigned long long I = u - J * (J + 1ull) / 2ull;
-    const uint32_t r0 = static_cast<uint32_t>(I) * kPotTile + tid, c0 = static_cast<uint32_t>(J) * kPotTile;
+    const uint32_t r0 = static_cast<uint32_t>(I) * kPotTile, c0 = static_cast<uint32_t>(J) * kPotTile;
     const uint32_t cnt = min(static_cast<uint32_t>(kPotTile), n - c0);
     double x[2], y[2], z[2], m[2], s[2] = {0.0, 0.0};
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const uint32_t i = r0 + k * kPotThreads;
+      const uint32_t i = r0 + row[k];
       x[k] = y[k] = z[k] = m[k] = 0.0;
       if (i < n) {
         x[k] = pos[3 * (size_t)i];
@@ -132,25 +125,27 @@ __global__ void __launch_bounds__(kPotThreads) k_potential_f64(uint32_t n, const
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           const double dx = c.x - x[k], dy = c.y - y[k], dz = c.z - z[k];
-          s[k] = fma(c.w, inv_sqrt(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)))), s[k]);
+          s[k] = fma(c.w, rsqrt(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)))), s[k]);
         }
       }
     } else {
-      for (uint32_t q = 0; q < cnt; ++q) {
-        const double4 c = src[q];
+      // only columns right of a row's own; the warp's other rows add nothing there (massless,
+      // at unit distance), and columns left of all of them are passed over
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          // only columns right of the row's own; the others add nothing (massless, at unit distance)
-          const bool on = q > static_cast<uint32_t>(tid + k * kPotThreads);
+      for (int k = 0; k < 2; ++k) {
+#pragma unroll 4
+        for (uint32_t q = (row[k] & ~31u) + 1u; q < cnt; ++q) {
+          const double4 c = src[q];
           const double dx = c.x - x[k], dy = c.y - y[k], dz = c.z - z[k];
+          const bool on = q > row[k];
           const double r2 = on ? fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))) : 1.0;
-          s[k] = fma(on ? c.w : 0.0, inv_sqrt(r2), s[k]);
+          s[k] = fma(on ? c.w : 0.0, rsqrt(r2), s[k]);
         }
       }
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k)
-      if (r0 + k * kPotThreads < n) total = fma(-g * m[k], s[k], total);
+      if (r0 + row[k] < n) total = fma(-g * m[k], s[k], total);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);

@@ -26,3 +26,20 @@ def test_extreme_distances(oracle):
     assert abs(s.potential_energy(pos, mass=mass) - ref) <= 1e-12 * abs(ref)
     pos[1] = pos[0]  # coincident, unsoftened: the pair's energy is infinite
     assert s.potential_energy(pos, mass=mass) == -np.inf
+
+
+def test_rounding_of_many_partial_sums():
+    # Against 80-bit sums. The terms' roundings average out over 4e7 pairs, so what is left is
+    # the last rounding (1.1e-16 at most) and the sum of the blocks' partials, which a plain
+    # sum rounds to 4.6e-16 on average and a compensated one not at all.
+    errors = []
+    for seed in range(3):
+        st = gb.ic.plummer(9000, seed)
+        p, m = st.pos.astype(np.longdouble), st.mass.astype(np.longdouble)
+        u = np.longdouble(0.0)
+        for i in range(0, 9000, 250):
+            d2 = ((p[i:i + 250, None, :] - p[None, i:, :]) ** 2).sum(axis=2) + np.longdouble(0.01 * 0.01)
+            w = m[i:i + 250, None] * m[None, i:] / np.sqrt(d2)
+            u -= np.triu(w, 1).sum()
+        errors.append(float(abs((gb.GpuLbvh(1.0, 0.01, 0.5).potential_energy(st) - u) / u)))
+    assert np.mean(errors) <= 2.0 ** -53, errors
