@@ -481,6 +481,7 @@ void enqueue_tree(gx_handle* h, const StepBufs& b, int kick, int pending, bool t
   {
     NvtxRange r("gx.build");
     launch_build(b, h->opt.multipole == GX_MULTIPOLE_QUAD && h->opt.precision != GX_PREC_F64, st);
+    if (h->opt.precision == GX_PREC_F64) launch_walk_records64(b, st);
   }
   if (timed) cudaEventRecord(h->ev[3], st);
 }

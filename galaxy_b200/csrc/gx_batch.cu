@@ -145,6 +145,7 @@ void enqueue_step(gx_batch* bt, int kick, bool inside) {
   launch_sort(b, st);
   const int quad = bt->opt.multipole == GX_MULTIPOLE_QUAD && bt->opt.precision != GX_PREC_F64;
   launch_build(b, quad, st);
+  if (bt->opt.precision == GX_PREC_F64) launch_walk_records64(b, st);
   launch_walk(b, bcfg(bt, inside), st);
 }
 

@@ -133,6 +133,8 @@ void launch_build(const StepBufs& b, int quad, cudaStream_t st);
 void build_prepare();
 // gx_walk.cu: tree walk, acc in original order
 void launch_walk(const StepBufs& b, const WalkCfg& cfg, cudaStream_t st);
+// the FP64 walk's records of a tree just built (kept with it: a cached tree's walks reuse them)
+void launch_walk_records64(const StepBufs& b, cudaStream_t st);
 // gx_diag.cu: one bounded wait on a word nothing sets (failure-detection self-test)
 void launch_selftest_wait(const uint32_t* word, uint32_t spins, DevCtl* ctl, cudaStream_t st);
 // gx_active.cu: the active-subset walk's target list. From the sorted order and the

@@ -82,7 +82,7 @@ __device__ __forceinline__ unsigned long long warp_sum64(unsigned long long v) {
 
 }  // namespace
 
-// The FP64 walk's records, one thread a sorted position: the internal node of that index
+// The FP64 walk's records, made once a tree, one thread a sorted position: the internal node of that index
 // and the leaf. The node after a subtree in depth-first order is the right child of the
 // first ancestor that the subtree lies to the left of, two steps up on average. The
 // thresholds bracket the reference's test theta (d - delta) >= s on d^2 by 1e-9 (its
@@ -1057,7 +1057,6 @@ void dispatch(const StepBufs& b, const WalkCfg& cfg, cudaStream_t st) {
   if (cfg.precision == 1) {
     // The FP64 walk has no quadrupole or compensation variants: it is the
     // reference's arithmetic.
-    if (b.ntiles) k_walk_records64<<<b.ntiles, kTileThreads, 0, st>>>(b);
     if (cfg.stats)
       launch_k(k_walk_f64<true, LIST>, b, cfg, 0, st);
     else
@@ -1117,6 +1116,10 @@ int walk_resident_ctas(const WalkCfg& cfg) {
   if (cfg.precision == 1) return resident(k_walk_f64<false, false>, block, 0);
   if (cfg.quad) return resident(k_walk_f32<true, true, false, false, false>, block, walk_smem_bytes(block, true));
   return resident(k_walk_f32<false, true, false, false, false>, block, walk_smem_bytes(block, false));
+}
+
+void launch_walk_records64(const StepBufs& b, cudaStream_t st) {
+  if (b.ntiles) k_walk_records64<<<b.ntiles, kTileThreads, 0, st>>>(b);
 }
 
 void launch_walk(const StepBufs& b, const WalkCfg& cfg, cudaStream_t st) {

@@ -83,3 +83,21 @@ def test_stale_walk_with_massless_leaves(oracle):
     s.rebuild_gravity_cache(pos0, mass=mass)
     got = s.gravity_active_cached(pos1, act, mass=mass)
     assert np.array_equal(got[act], oracle.lbvh_accelerations_stale(pos0, mass, pos1, mass, G, EPS, 0.5, act))
+
+
+def test_f64_walk_of_one_target_does_not_grow_with_the_tree():
+    # The FP64 walk's records belong to the tree, so that walks of a cached tree reuse them:
+    # the walk stage of one target at a wide opening angle hardly depends on the tree's size.
+    # (Records made in every walk: 103 and 325 us at 2^14 and 2^22 particles; with the tree: 48
+    # and 118 us.)
+    ms = []
+    for n in (1 << 14, 1 << 22):
+        rng = np.random.default_rng(n)
+        pos, mass, out = rng.random((n, 3)), np.full(n, 1.0 / n), np.zeros((n, 3))
+        s = gb.GpuLbvh(1.0, 0.02, 3.0, precision="f64", stage_times=True)
+        t = []
+        for _ in range(8):
+            s.accelerations_active(pos, [n // 2], out, mass=mass)
+            t.append(s.stats()["ms_walk"])
+        ms.append(min(t))
+    assert ms[1] <= ms[0] + 0.14, ms
