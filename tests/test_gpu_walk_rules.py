@@ -54,3 +54,19 @@ def test_list_edges_quad(oracle, n):
         got = gb.GpuLbvh(1.0, 0.05, 0.6, multipole="quad", walk_group=group).accelerations(pos, mass=mass)
         err = oracle.per_particle_rel_err(got, ref)
         assert np.median(err) <= 1e-6 and np.percentile(err, 99) <= 1e-5
+
+
+@pytest.mark.parametrize("theta", [0.0, 1e-300, 1e-3, 1.1499, 1.15, 1.1547, 1.2, 2.0, 5.0, 40.0, 1e9, np.inf])
+@pytest.mark.parametrize("scale", [1.0, 1e-60, 1e-75, 1e60, 1e71])
+def test_fp64_thresholds(oracle, theta, scale):
+    # the FP64 walk's squared-distance thresholds: open everything, beyond the box's corners
+    # where the inside rule binds, and squares that leave the range of a double
+    pos, _, mass = oracle.fixture_cluster(4, 700)
+    pos[:150, 2] = 0.0
+    pos[150:200, 1:] = 0.25
+    pos[200:220] = pos[200]
+    mass[300:330] = 0.0
+    pos = pos * scale
+    got = gb.GpuLbvh(1.0, 0.0 if scale == 1.0 else 0.05 * scale, theta, precision="f64").accelerations(pos, mass=mass)
+    ref = oracle.lbvh_accelerations(pos, mass, 1.0, 0.0 if scale == 1.0 else 0.05 * scale, theta, threads=THREADS)
+    assert np.array_equal(got, ref, equal_nan=True)
