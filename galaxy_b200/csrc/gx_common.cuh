@@ -129,6 +129,15 @@ struct TileDesc {
   uint32_t sys, begin, end, pad;
 };
 
+// The part of tile blockIdx.x / split that this block takes, [begin, end).
+__device__ __forceinline__ TileDesc tile_part(const TileDesc* __restrict__ tiles, int split) {
+  TileDesc t = tiles[blockIdx.x / split];
+  const uint32_t len = kTile / split;
+  t.begin += (blockIdx.x % split) * len;
+  t.end = min(t.end, t.begin + len);
+  return t;
+}
+
 // One independent particle system (a batch holds many, packed back to back).
 struct SysDesc {
   uint32_t off, n;              // particle range [off, off + n)

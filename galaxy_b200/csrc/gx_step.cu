@@ -39,15 +39,6 @@ __device__ __forceinline__ void block_bbox_commit(double v[6], unsigned long lon
 
 }  // namespace
 
-// The part of tile blockIdx.x / split that this block takes, [begin, end).
-__device__ __forceinline__ TileDesc tile_part(const TileDesc* __restrict__ tiles, int split) {
-  TileDesc t = tiles[blockIdx.x / split];
-  const uint32_t len = kTile / split;
-  t.begin += (blockIdx.x % split) * len;
-  t.end = min(t.end, t.begin + len);
-  return t;
-}
-
 // `split` CTAs per tile. kick: apply the (deferred closing +) opening half kick and the
 // drift before reducing the bounding box of the new positions.
 //   pending:  v += a*h   (closing half kick of the previous step, kept separate)
@@ -331,12 +322,7 @@ void run_small(const StepBufs& b, cudaStream_t st) {
                b.bounds, reinterpret_cast<K*>(b.codes), b.order);
 }
 
-// CTAs per tile of the streaming kernels: a tile a CTA leaves most SMs idle, and 16 particles
-// a thread one after another, until there are a few tiles per SM. The histogram kernel
-// pays one merge of its bins per CTA, so it splits less.
-// Measured (kick + bbox and Morton together, us): 4,096 particles 36 -> 18, 65,536 36 ->
-// 20, 200,003 38 -> 23, 600,000 42 -> 37.
-int stream_split(uint32_t ntiles) { return ntiles <= 74 ? 16 : ntiles <= 296 ? 4 : 1; }
+// The histogram kernel pays one merge of its bins per CTA, so it splits less than stream_split.
 int hist_split(uint32_t ntiles) { return ntiles <= 37 ? 8 : ntiles <= 148 ? 4 : 1; }
 
 }  // namespace
