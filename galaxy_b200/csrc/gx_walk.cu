@@ -140,6 +140,29 @@ __global__ void __launch_bounds__(kTileThreads) k_walk_records64(StepBufs b, int
   }
 }
 
+namespace {
+
+// Nodes that the walks of a warp's targets visit, each counted once (the statistic
+// warp_node_visits): the warp goes through the tree in depth-first order, and a lane waits
+// until the warp is at the next node of its own walk.
+__device__ __noinline__ uint32_t warp_visits(const StepBufs& b, const SysDesc& sd, const double x[3], bool valid) {
+  const uint32_t n_total = b.n, int_lo = n_total + sd.off, max_steps = 2u * sd.n;
+  uint32_t mine = valid ? int_lo : kWalkEnd, count = 0;
+  uint32_t u = __any_sync(0xffffffffu, valid) ? int_lo : kWalkEnd;
+  while (count < max_steps && (u - sd.off < sd.n || u - int_lo < sd.n - 1u)) {
+    ++count;
+    const bool leaf = u < n_total, at = mine == u;
+    const uint32_t next = leaf ? b.leaf_next[u] : b.rec64[u - n_total].next;
+    const uint32_t left = leaf ? kWalkEnd : b.rec64[u - n_total].left;
+    const bool open = at && !leaf && exact_decision(b.agg64, u - n_total, x, sd.theta) == 0;
+    if (at) mine = open ? left : next;
+    u = __any_sync(0xffffffffu, open) ? left : next;
+  }
+  return count;
+}
+
+}  // namespace
+
 // Exact FP64 walk: every lane walks the tree for its own target in strict depth-first,
 // left-before-right order and adds its terms in that order with the reference's arithmetic.
 // A record names its successor for either decision, so there is no stack, and the next
@@ -164,7 +187,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_f64(StepBufs b, int persi
     const bool valid = LIST ? (lane < static_cast<int>(b.group) && li < *b.ntargets) : li < end;
     const uint32_t k = LIST ? (valid ? b.targets[li] : 0u) : li;
     double a64[3] = {0.0, 0.0, 0.0};
-    unsigned long long n_leaf = 0, n_far = 0, n_open = 0, n_vis = 0;
+    unsigned long long n_leaf = 0, n_far = 0, n_open = 0;
     if (sd.n > 1 && valid) {
       const double eps2 = dmul(sd.eps, sd.eps);
       const double4 x = b.leaf64[k];
@@ -198,7 +221,6 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_f64(StepBufs b, int persi
           raise_err(b.ctl, kErrBadIndex);
           break;
         }
-        if (STATS) ++n_vis;
         const double dx = dsub(p.x, x3[0]), dy = dsub(p.y, x3[1]), dz = dsub(p.z, x3[2]);
         const double d2 = dlen2(dx, dy, dz);
         const double m = p.w;
@@ -242,15 +264,17 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_f64(StepBufs b, int persi
       for (int c = 0; c < 3; ++c) b.acc[3 * (size_t)o + c] = sd.n > 1 ? dmul(a64[c], sd.g) : 0.0;
     }
     if (STATS) {
+      const double4 xv = valid ? b.leaf64[k] : make_double4(0.0, 0.0, 0.0, 0.0);
+      const double x3[3] = {xv.x, xv.y, xv.z};
+      const uint32_t n_vis = sd.n > 1 ? warp_visits(b, sd, x3, valid) : 0u;
       n_leaf = warp_sum64(n_leaf);
       n_far = warp_sum64(n_far);
       n_open = warp_sum64(n_open);
-      n_vis = warp_sum64(n_vis);
       if (lane == 0) {
         atomicAdd(&b.ctl->stats[0], n_leaf);
         atomicAdd(&b.ctl->stats[1], n_far);
         atomicAdd(&b.ctl->stats[2], n_open);
-        atomicAdd(&b.ctl->stats[4], n_vis);
+        atomicAdd(&b.ctl->stats[4], static_cast<unsigned long long>(n_vis));
       }
     }
     if (persistent) {

@@ -81,7 +81,8 @@ typedef struct gx_stats {
   uint64_t far_interactions;
   uint64_t nodes_opened;
   uint64_t f64_rechecks;   /* opening decisions re-evaluated in FP64 (guard band) */
-  uint64_t warp_node_visits;
+  uint64_t warp_node_visits; /* tree records read by the walk's warps, each counted once a warp:
+                                nodes (leaves included) in FP64, pairs of siblings in FP32 */
   float ms_bbox_morton;    /* stage times of the last call, CUDA events */
   float ms_sort;
   float ms_build;

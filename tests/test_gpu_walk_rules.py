@@ -70,3 +70,19 @@ def test_fp64_thresholds(oracle, theta, scale):
     got = gb.GpuLbvh(1.0, 0.0 if scale == 1.0 else 0.05 * scale, theta, precision="f64").accelerations(pos, mass=mass)
     ref = oracle.lbvh_accelerations(pos, mass, 1.0, 0.0 if scale == 1.0 else 0.05 * scale, theta, threads=THREADS)
     assert np.array_equal(got, ref, equal_nan=True)
+
+
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 100, 700])
+def test_warp_node_visits(oracle, n):
+    # At theta 0 every target goes through the whole tree: a warp's visits are the tree's nodes
+    # (FP64, 32 targets a warp) or its sibling pairs (FP32), each counted once a warp.
+    pos, _, mass = oracle.fixture_cluster(n, n)
+    kw = dict(stats=True)
+    s = gb.GpuLbvh(1.0, 0.05, 0.0, precision="f64", **kw)
+    ref = oracle.lbvh_accelerations(pos, mass, 1.0, 0.05, 0.0, threads=THREADS)
+    assert np.array_equal(s.accelerations(pos, mass=mass), ref)
+    assert s.stats()["warp_node_visits"] == -(-n // 32) * (2 * n - 1)
+    for group in (8, 16, 32):
+        s = gb.GpuLbvh(1.0, 0.05, 0.0, walk_group=group, **kw)
+        s.accelerations(pos, mass=mass)
+        assert s.stats()["warp_node_visits"] == -(-n // group) * (n - 1)
