@@ -343,7 +343,8 @@ struct gx_handle {
   bool pending_kick = false;
   uint64_t launches = 0;
   gx_stats stats{};
-  // every tree build bumps tree_gen; the stale-tree cache is valid while it holds
+  // what builds a tree, or writes over one or its numbering, bumps tree_gen; the stale-tree
+  // cache is valid while it holds
   uint64_t tree_gen = 0, cache_gen = ~0ull;
   size_t cache_n = 0;
   // active-subset walk (gx_accelerations_active): buffers grown on demand
@@ -414,6 +415,7 @@ int layout(gx_handle* h, size_t n, double dt) {
       system_walk_group(h->device, h->opt, n) == h->group_layout &&
       static_cast<int>(system_radix_bits(h->device, h->opt, n)) == h->ar.b.radix_bits)
     return GX_OK;
+  if (n != h->n_layout) ++h->tree_gen;  // its nodes are numbered, and its buffers sized, by n
   std::vector<SysDesc> in(1), sys;
   in[0].off = 0;
   in[0].n = static_cast<uint32_t>(n);
@@ -1381,6 +1383,7 @@ int gx_stage_morton(gx_handle* h, size_t n, const double* pos, uint32_t* lanes_o
   GX_CK(h, copy_in(h->device, h->stream, b.pos, pos, 3 * n * sizeof(double)));
   GX_CK(h, cudaMemsetAsync(b.zero_begin, 0, b.zero_bytes, h->stream));
   launch_kick_drift_bbox(b, 0, 0, h->stream);
+  ++h->tree_gen;
   // Lanes (3n u32) are staged in the walk records, unused by this stage.
   uint32_t* d_lanes = lanes_out ? reinterpret_cast<uint32_t*>(b.pairs) : nullptr;
   launch_morton_hist(b, d_lanes, h->stream);
@@ -1414,6 +1417,7 @@ int gx_stage_sort(gx_handle* h, size_t n, const uint32_t* codes, uint32_t* order
   StepBufs& b = h->ar.b;
   GX_CK(h, cudaMemcpyAsync(b.codes, codes, n * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
   GX_CK(h, cudaMemsetAsync(b.zero_begin, 0, b.zero_bytes, h->stream));
+  ++h->tree_gen;
   launch_code_hist(b, h->stream);
   launch_sort(b, h->stream);
   GX_CK(h, cudaMemcpyAsync(order_out, b.order, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
@@ -1445,6 +1449,7 @@ int gx_stage_build(gx_handle* h, size_t n, const uint32_t* sorted_codes, const d
   const int quad = h->opt.multipole == GX_MULTIPOLE_QUAD && h->opt.precision != GX_PREC_F64;
   GX_CK(h, cudaMemsetAsync(b.bounds, 0, sizeof(Bounds), h->stream));  // no Morton stage here
   GX_CK(h, cudaMemsetAsync(b.slots, 0xFF, n * sizeof(unsigned long long), h->stream));  // nor the kick's arming
+  ++h->tree_gen;
   launch_build(b, quad, h->stream);
   std::vector<uint2> kids(n > 1 ? n - 1 : 1);
   std::vector<Agg64> agg(n > 1 ? n - 1 : 1);

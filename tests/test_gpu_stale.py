@@ -101,3 +101,32 @@ def test_f64_walk_of_one_target_does_not_grow_with_the_tree():
             t.append(s.stats()["ms_walk"])
         ms.append(min(t))
     assert ms[1] <= ms[0] + 0.14, ms
+
+
+@pytest.mark.parametrize("other", ["potential of more", "potential of fewer", "direct sum", "morton", "sort", "build"])
+def test_cache_is_refused_once_its_buffers_are_written(oracle, other):
+    # Calls that build no walkable tree of their own but size the handle's buffers for another
+    # number of particles, or write over the cached tree's.
+    pos, _, mass = oracle.fixture_cluster(44, 2000)
+    big, _, bmass = oracle.fixture_cluster(45, 9000)
+    s = gb.GpuStaleTreeGravity(G, EPS, 0.5)
+    s.rebuild_gravity_cache(pos, mass=mass)
+    want = s.gravity_active_cached(pos, [1, 2, 3], mass=mass)
+    s.potential_energy(pos, mass)  # as many particles: the cache stays
+    assert np.array_equal(s.gravity_active_cached(pos, [1, 2, 3], mass=mass), want)
+    if other == "potential of more":
+        s.potential_energy(big, bmass)
+    elif other == "potential of fewer":
+        s.potential_energy(pos[:900], mass[:900])
+    elif other == "direct sum":
+        s.direct_sum_f64(big, bmass, targets=[0, 1])
+    elif other == "morton":
+        gb.stage_morton(pos, handle=s)
+    elif other == "sort":
+        gb.stage_sort(np.arange(2000, dtype=np.uint32), handle=s)
+    else:
+        gb.stage_build(np.arange(2000, dtype=np.uint32), pos, mass, handle=s)
+    with pytest.raises(gb.GxError):
+        s.gravity_active_cached(pos, [1, 2, 3], mass=mass)
+    s.rebuild_gravity_cache(pos, mass=mass)
+    assert np.array_equal(s.gravity_active_cached(pos, [1, 2, 3], mass=mass), want)
