@@ -86,3 +86,27 @@ def test_warp_node_visits(oracle, n):
         s = gb.GpuLbvh(1.0, 0.05, 0.0, walk_group=group, **kw)
         s.accelerations(pos, mass=mass)
         assert s.stats()["warp_node_visits"] == -(-n // group) * (n - 1)
+
+
+def test_targets_across_a_morton_jump(oracle):
+    # Groups of targets from tight clumps either side of the cube's middle planes: their boxes
+    # are wide, and clumps that are undecided for a group lie close to some of its targets.
+    # Coordinates relative to the box's centre would lose bits (largest error of a particle
+    # 4e-5 at least in each of these walks); the near list keeps them (7.8e-6 at most, which is
+    # that of entries accepted for the whole group).
+    n = 8000
+    rng = np.random.default_rng(11)
+    c = (rng.integers(0, 2, (n, 3)) - 0.5) * 2e-4 * rng.uniform(0.1, 1, (n, 1))
+    pos = c + rng.normal(size=(n, 3)) * 2e-5
+    pos[::9] = rng.uniform(-1, 1, pos[::9].shape)
+    mass = rng.uniform(0.5, 1.5, n) / n
+    ref = gb.GpuLbvh(1.0, 0.02, 0.7, precision="f64", morton63=True).accelerations(pos, mass=mass)
+    size = np.linalg.norm(ref, axis=1)
+    act = np.sort(np.random.default_rng(1).choice(n, n // 50, replace=False)).astype(np.int64)
+    for group in (8, 16, 32):
+        s = gb.GpuLbvh(1.0, 0.02, 0.7, morton63=True, walk_group=group)
+        err = np.linalg.norm(s.accelerations(pos, mass=mass) - ref, axis=1) / size
+        assert err.max() <= 2e-5, (group, err.max())
+    got = s.accelerations_active(pos, act, mass=mass)[act]
+    err = np.linalg.norm(got - ref[act], axis=1) / size[act]
+    assert err.max() <= 2e-5, err.max()
