@@ -71,11 +71,13 @@ constexpr int kWalkCtas = 4, kWalkCtasQuad = 4;
 
 // Launches kern after the kernel before it on st, to be scheduled as that one drains; kern
 // begins with step_kernel_begin. That takes about 1 us off the gap to the kernel before
-// it (a step of 16,384 particles: codes, sort and build 161 -> 148 us). From kEarlyTiles
-// tiles on it is an ordinary launch: blocks placed while the kernel before still runs land
-// unevenly, which costs what the gap gains (24 systems, 104 tiles: 0.7% slower; the tree
-// walk, whose blocks run longest, up to 4%, so it never is launched early).
-constexpr uint32_t kEarlyTiles = 80;
+// it. Above kEarlyTiles tiles it is an ordinary launch: blocks placed while the kernel before
+// still runs land unevenly, which costs more than the gap (and more yet in the tree walk,
+// whose blocks run longest: up to 4%, so it never is launched early). A step of a disk, us,
+// ordinary / early: 2 tiles 222.8 / 214.7, 4 246.2 / 239.5, 8 311.6 / 309.1, 12 368.5 / 366.6,
+// 14 388.1 / 385.7, 16 427.2 / 432.1, 24 464.9 / 467.4, 48 700.9 / 710.6, 64 863 / 878, 80 1037 /
+// 1064; 16 systems of a tile 342.7 / 352.5, 40 of two 1010 / 1037.
+constexpr uint32_t kEarlyTiles = 12;
 template <class... P, class... A>
 void launch_after(uint32_t ntiles, void (*kern)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute attr;
