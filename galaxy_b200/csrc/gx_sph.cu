@@ -26,7 +26,7 @@
 // covers its ball). One warp serves one target: its lanes walk the query box's buckets
 // 32 at a time as one flattened list. The density warp keeps its candidates (radius,
 // sorted slot) in shared memory and evaluates counts from there (streaming
-// the box again only when more than kCandCap candidates fall inside). It gathers a ball
+// the box again only when more candidates than its cache holds fall inside). It gathers a ball
 // of 2.1 to 2.5 x the bracket seed instead of the reference's 2 x hi = 4 x seed: a comparison
 // whose count needs a wider ball is settled by the lower bound of the gathered part when
 // that clears n_ngb, else the gather widens first, so every comparison is the reference's.
@@ -51,7 +51,16 @@ constexpr int kSphThreads = 128;                  // one target per warp
 constexpr int kSphWarps = kSphThreads / 32;
 constexpr int kDensThreads = 256;                 // density: one target per warp, 8 a block
 constexpr int kDensWarps = kDensThreads / 32;
-constexpr int kCandCap = 256;                     // density candidates cached per warp (512 and three blocks an SM: 8% slower)
+// Density candidates cached per warp, and the neighbour numbers that take the larger cache. A
+// cold ball of 2.5 seeds holds about 2 n_ngb particles, a warm one of 2.1 h 1.2 n_ngb; the
+// larger cache leaves three blocks an SM instead of four. Density of a cube / disk of 100,000,
+// cold, then warm, us, smaller / larger cache: n_ngb 48 2704 / 2789, 8287 / 9430, 2389 / 2496,
+// 3736 / 4498; 128 3750 / 3179, 18724 / 17114, 2657 / 2791, 6189 / 7539; 160 8853 / 3328,
+// 38918 / 19618, 2835 / 2866, 9796 / 8861; 300 11435 / 9766, 41981 / 32333, 5901 / 3303, 16154 /
+// 10130; 400 (a sphere of 30,000 too) 12250 / 11591, 32192 / 37748, 7133 / 4748, 9278 / 9990; 600
+// 13632 / 13672, 62633 / 66370, 8306 / 8985, 24054 / 28178.
+constexpr int kCandCap = 256, kCandCapWide = 512;
+constexpr double kWideNgbAbove = 128.0, kWideNgbMost = 350.0;
 constexpr double kLowerBoundMargin = 1.0 + 1e-10; // a partial count this far above n_ngb decides
 constexpr double kSureMargin = 1e-11;             // a count this far from n_ngb settles its side
 constexpr int kPairCap = 128;                     // hydro: neighbour slots listed per warp
@@ -443,9 +452,10 @@ struct DensArgs {
   const uint32_t* inv;      // gas-local index -> slot of this grid
 };
 
-__global__ void __launch_bounds__(kDensThreads, 4) k_sph_density(DensArgs a) {
-  __shared__ double s_r[kDensWarps][kCandCap];
-  __shared__ uint32_t s_s[kDensWarps][kCandCap];
+template <int CAP>
+__global__ void __launch_bounds__(kDensThreads, CAP <= kCandCap ? 4 : 3) k_sph_density(DensArgs a) {
+  __shared__ double s_r[kDensWarps][CAP];
+  __shared__ uint32_t s_s[kDensWarps][CAP];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t w = blockIdx.x * kDensWarps + warp;
   if (w >= (a.targets ? a.n_targets : a.g.n)) return;  // warp-uniform
@@ -485,13 +495,13 @@ __global__ void __launch_bounds__(kDensThreads, 4) k_sph_density(DensArgs a) {
       }
       const unsigned m = __ballot_sync(kFull, in);
       const uint32_t at = ncand + __popc(m & ((1u << lane) - 1u));
-      if (in && at < static_cast<uint32_t>(kCandCap)) {
+      if (in && at < static_cast<uint32_t>(CAP)) {
         cr[at] = r2;
         cs[at] = s;
       }
       ncand += __popc(m);
     });
-    over = ncand > static_cast<uint32_t>(kCandCap);
+    over = ncand > static_cast<uint32_t>(CAP);
     __syncwarp();
     if (!over) {  // the distances, one pass with every lane busy
       for (uint32_t j = lane; j < ncand; j += 32) cr[j] = sqrt(cr[j]);
@@ -1243,7 +1253,10 @@ void sph_enqueue_force(SphState& s, const double* pos, const double* vel, const 
     da.n_targets = n_targets;
     da.inv = s.grid[1].inv;
     const uint32_t nd = targets ? n_targets : n;
-    if (nd) k_sph_density<<<(nd + kDensWarps - 1) / kDensWarps, kDensThreads, 0, st>>>(da);
+    const bool wide = da.n_ngb > kWideNgbAbove && da.n_ngb <= kWideNgbMost;
+    const uint32_t blocks = (nd + kDensWarps - 1) / kDensWarps;
+    if (nd && wide) k_sph_density<kCandCapWide><<<blocks, kDensThreads, 0, st>>>(da);
+    if (nd && !wide) k_sph_density<kCandCap><<<blocks, kDensThreads, 0, st>>>(da);
   }
   if (after_density) cudaEventRecord(after_density, st);
   if (!hydro) {

@@ -65,3 +65,36 @@ def test_far_outliers_cost_about_as_much():
         return min(t)
 
     assert best(far) <= 4.0 * best(pos)
+
+
+def test_cost_where_a_cold_ball_outgrows_the_smaller_cache():
+    # 200 neighbours: a cold ball of about 400 candidates is cached whole, not streamed again
+    # for every count. The cold solve then takes 1.2 times as long as the warm one, 2.4 times
+    # when it streams.
+    import time
+
+    rng = np.random.default_rng(5)
+    pos, mass = rng.random((100_000, 3)), np.full(100_000, 1e-5)
+    s = gb.GpuGravitySph(1.0, 0.01, 0.5, sph=dict(n_ngb=200.0))
+    _, h = s.density(pos, mass)
+
+    def best(hint):
+        t = []
+        for _ in range(8):
+            t0 = time.perf_counter()
+            s.density(pos, mass, hint)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    assert best(None) <= 1.8 * best(h)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "core"])
+@pytest.mark.parametrize("n_ngb", [128.0, 129.0, 350.0, 351.0])
+def test_h_at_the_edges_of_the_cache_rule(oracle, kind, n_ngb):
+    rng = np.random.default_rng(7)
+    pos, mass = _cloud(kind, 3000, rng), rng.uniform(0.5, 1.0, 3000)
+    rho, h = gb.GpuGravitySph(1.0, 0.01, 0.5, sph=dict(n_ngb=n_ngb)).density(pos, mass)
+    ref_rho, ref_h = oracle.sph_density_adaptive(pos, mass, n_ngb=n_ngb)
+    assert np.allclose(h, ref_h, rtol=1e-12, atol=0.0)
+    assert np.allclose(rho, ref_rho, rtol=1e-11, atol=0.0)
