@@ -7,15 +7,16 @@
 // between the staging buffer and the caller's array. Measured, us, through the driver / this
 // way: inputs of 400 KB 34 / 32, 1 MB 68 / 52, 12 MB 640 / 410; outputs of 100 KB 23 / 19,
 // 1 MB 90 / 49, 12 MB 720 / 336; 50 MB into new arrays 23,800 / 5,100. Arrays that are pinned
-// already, and copies below kMinIn and kMinOut, go directly.
+// already, and inputs below kMinIn, go directly.
 //
 // Making it ready costs more than a short program gains: 8 MB of pinned memory take 5 ms (4 KB
 // take 2), a thread's team of 8 about 0.8 ms. So a thread's copies go directly until it has
-// copied kCredit bytes (a larger copy is staged at once: its page faults alone cost more), and
-// the last staging buffer outlives the handles, so that programs which make a handle a call
-// pay once. First call of a program's only handle, us, through the driver / with the buffer
-// made in each handle's first call / this way: 2,000 particles 767 / 5,590 / 700; 200,003
-// 7,780 / 13,750 / 7,010. 50,000 particles in 8 threads of 3 calls each: 1,550 / 2,520 / 1,360.
+// copied kCredit bytes (an output counts as kOutCredit at least; a larger copy is staged at
+// once: its page faults alone cost more), and the last staging buffer outlives the handles,
+// so that programs which make a handle a call pay once. First call of a program's only
+// handle, us, through the driver / with the buffer made in each handle's first call / this
+// way: 2,000 particles 767 / 5,590 / 700; 200,003 7,780 / 13,750 / 7,010. 50,000 particles in
+// 8 threads of 3 calls each: 1,550 / 2,520 / 1,360.
 //
 // A staging buffer belongs to one call at a time. There are at most kMaxBuffers; with all of
 // them in use a copy goes directly.
@@ -33,7 +34,7 @@ namespace {
 constexpr size_t kSlot = size_t{1} << 20;
 constexpr int kSlots = 8;
 constexpr size_t kMinIn = size_t{1} << 19;
-constexpr size_t kMinOut = size_t{1} << 17;
+constexpr size_t kOutCredit = size_t{1} << 17;
 constexpr size_t kCredit = size_t{32} << 20;
 constexpr size_t kPiece = size_t{1} << 17;  // bytes a thread moves at a time
 constexpr int kMaxBuffers = 4;
@@ -52,9 +53,8 @@ int g_made = 0;  // idle or in use
 size_t g_users = 0;
 thread_local size_t t_copied = 0;
 
-// Whether a copy of this many bytes is staged; counts it towards the thread's credit.
-bool staged(size_t bytes, size_t least) {
-  if (bytes < least) return false;
+// Whether a copy is staged, counting it as so many bytes towards the thread's credit.
+bool staged(size_t bytes) {
   if (t_copied <= kCredit) t_copied += std::min(bytes, kCredit + 1);
   return t_copied > kCredit;
 }
@@ -160,7 +160,7 @@ void transfer_unref() {
 }
 
 cudaError_t copy_in(int device, cudaStream_t st, void* dst, const void* src, size_t bytes) {
-  Staging* s = bytes >= kMinIn && pageable(src) && staged(bytes, kMinIn) ? acquire(device) : nullptr;
+  Staging* s = bytes >= kMinIn && pageable(src) && staged(bytes) ? acquire(device) : nullptr;
   if (!s) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
   cudaError_t e = cudaSuccess;
   int k = 0;
@@ -218,7 +218,7 @@ cudaError_t copy_out(int device, cudaStream_t st, const HostPiece* pieces, int c
       total += pieces[i].bytes;
     }
   char* to = total && total <= kSmallOut ? small : nullptr;  // all of them go through `small`
-  Staging* s = !to && total && staged(total, kMinOut) ? acquire(device) : nullptr;
+  Staging* s = !to && total && staged(std::max(total, kOutCredit)) ? acquire(device) : nullptr;
   for (int i = 0; i < count && e == cudaSuccess; ++i) {
     const HostPiece& p = pieces[i];
     if (!p.host || !p.bytes) continue;
