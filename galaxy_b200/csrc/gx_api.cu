@@ -203,8 +203,6 @@ cudaError_t Arena::ensure(size_t n, size_t tiles, size_t items, size_t nsys, int
   diag_cap = nn / 256 + 2;
   GX_A(diag_partial, 8 * diag_cap, double);
 #undef GX_A
-  e = cudaMemsetAsync(b.slots, 0xFF, nn * sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(b.ctl, 0, sizeof(DevCtl), st);
   if (e != cudaSuccess) return e;
   cap_n = nn;
@@ -533,8 +531,7 @@ int finish(gx_handle* h, bool timed, const HostPiece* outs = nullptr, int n_outs
   h->stats.f64_rechecks = ctl.stats[3];
   h->stats.warp_node_visits = ctl.stats[4];
   if (ctl.err) {
-    // Re-arm the climb slots and clear the word so the handle stays usable.
-    cudaMemset(h->ar.b.slots, 0xFF, h->ar.cap_n * sizeof(unsigned long long));
+    // Clear the word so the handle stays usable (each step arms its climb slots).
     cudaMemset(h->ar.b.ctl, 0, sizeof(DevCtl));
     char buf[128];
     snprintf(buf, sizeof buf, "device check tripped (error word 0x%x)", ctl.err);

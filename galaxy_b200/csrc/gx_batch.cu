@@ -155,7 +155,6 @@ int bfinish(gx_batch* bt) {
   DevCtl ctl;
   GB_CK(bt, cudaMemcpy(&ctl, bt->ar.b.ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost));
   if (ctl.err) {
-    cudaMemset(bt->ar.b.slots, 0xFF, bt->ar.cap_n * sizeof(unsigned long long));
     cudaMemset(bt->ar.b.ctl, 0, sizeof(DevCtl));
     return bfail(bt, GX_ERR_DEVICE_CHECK, "device check tripped (error word " + std::to_string(ctl.err) + ")");
   }

@@ -50,8 +50,7 @@ constexpr double kOpenBand = 4e-6;
 
 // Device error word bits (read back by the host after each call).
 constexpr uint32_t kErrLookbackTimeout = 1u << 0;
-constexpr uint32_t kErrStackOverflow = 1u << 1;
-constexpr uint32_t kErrBadIndex = 1u << 2;
+constexpr uint32_t kErrBadIndex = 1u << 2;  // also a walk beyond its stack or its budget (bit 1 is free)
 constexpr uint32_t kErrClimb = 1u << 3;
 constexpr uint32_t kErrSphIterations = 1u << 4;  // an SPH root-find ran past its iteration bound
 

@@ -29,27 +29,6 @@ namespace gx {
 
 namespace {
 
-
-struct Acc32 {
-  float s[3], c[3];
-};
-
-template <bool KAHAN>
-__device__ __forceinline__ void acc_add(Acc32& a, float tx, float ty, float tz) {
-  const float t[3] = {tx, ty, tz};
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    if (KAHAN) {
-      const float y = __fsub_rn(t[i], a.c[i]);
-      const float u = __fadd_rn(a.s[i], y);
-      a.c[i] = __fsub_rn(__fsub_rn(u, a.s[i]), y);
-      a.s[i] = u;
-    } else {
-      a.s[i] += t[i];
-    }
-  }
-}
-
 // The reference's decision for internal node gi (solvers/src/lbvh.rs:485-514) in f64
 // on the node's f64 aggregate, geometry derived as in reference_flatten
 // (lbvh.rs:602-613): 1 = take the monopole, 0 = open, -1 = skip (massless subtree).
