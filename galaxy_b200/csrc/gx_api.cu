@@ -774,10 +774,13 @@ int walk_active(gx_handle* h, size_t n, size_t n_active, const uint32_t* active,
   const uint32_t na = static_cast<uint32_t>(n_active);
   uint32_t* count = a.chunks + active_chunk_count(static_cast<uint32_t>(n)) + 1;
   // Targets per warp: a sparse subset spreads 32 consecutive active targets over a wide
-  // region (a large union walk), so fewer lanes take part the sparser it is. Thresholds
-  // from a sweep on the 2^20 collision (walk ms at 0.3% / 1% / 3% / 10% / 30% active:
-  // 4 lanes 3.3 / 3.0 / 3.6 / 6.9 / 16.0, 8 lanes 4.2 / 3.2 / 3.2 / 5.1 / 9.8, 32 lanes
-  // 8.0 / 5.4 / 3.8 / 3.8 / 5.3; the full walk takes 9.5).
+  // region (a large union walk), so fewer lanes take part the sparser it is. The lines were
+  // drawn for an earlier walk; the present one would take narrower groups longer (walk us at
+  // 1% / 2% / 5% / 8% / 30% active, collision of 2^20: 4 targets 536 / 632 / 1025 / 1342 / 3679, 8
+  // 620 / 722 / 964 / 1093 / 2563, 16 1048 / 929 / 931 / 1191 / 2141, 32 2644 / 1416 / 1299 / 1301 /
+  // 2268; disk of 300,007: 4 300 / 255 / 357 / 441 / 1043, 8 353 / 316 / 316 / 411 / 765, 16 488 / 417 /
+  // 398 / 419 / 697, 32 855 / 704 / 638 / 689 / 771), but the grouping sets the last bits of the
+  // results, so they stay.
   const double frac = static_cast<double>(n_active) / static_cast<double>(n);
   // The FP64 walk's lanes walk by themselves, so it always fills its warps.
   const uint32_t group = h->opt.precision == GX_PREC_F64 || frac >= 0.08 ? 32u : frac >= 0.04 ? 16u : frac >= 0.015 ? 8u : 4u;

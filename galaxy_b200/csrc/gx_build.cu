@@ -309,8 +309,9 @@ struct BuildSmem {
 // unified index | left-child bit 31, far end of its range), the count at
 // vals_alt[first] -- so no block contends for a global counter.
 // A round: (A) every node completed in the last round (leaves in round 0) stages its
-// records and meets its sibling; (B) the second arrivals, compacted into the first
-// threads of the block, fold their parents. Half of the climbers leave at every level,
+// aggregate and meets its sibling; (B) the second arrivals are compacted into the first
+// threads of the block, which fold their parents, while the second half of the block stages
+// the walk records and links of the same parents. Half of the climbers leave at every level,
 // so compacting them keeps the FP64 folds in full warps; staging the records keeps the
 // rounds free of scattered global stores. No thread waits on another except at the
 // block's barriers.

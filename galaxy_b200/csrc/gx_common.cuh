@@ -84,8 +84,9 @@ struct Bounds {
   uint32_t pad;
 };
 
-// Work is cut into tiles of kTile particles that never straddle two systems; the
-// bbox, Morton, sort and build kernels each run one CTA per tile.
+// Work is cut into tiles of kTile particles that never straddle two systems. A sort pass
+// runs one CTA per tile, the build's first pass kTile / kBuildLeaves, the streaming kernels (kick
+// and bbox, Morton codes, FP64 walk records) up to 16 for few tiles.
 constexpr int kTile = 4096;
 constexpr int kTileThreads = 256;
 // Threads per block of the tree walks (and the largest walk block accepted).

@@ -117,10 +117,11 @@ struct WalkCfg {
 void launch_kick_drift_bbox(const StepBufs& b, int kick, int pending, cudaStream_t st);
 void launch_kick_half(const StepBufs& b, cudaStream_t st);
 void launch_morton_hist(const StepBufs& b, uint32_t* lanes_out, cudaStream_t st);
-// gx_sort.cu: the four onesweep passes (codes, iota) -> (codes sorted, order)
+// gx_sort.cu: the onesweep passes (codes, iota) -> (codes sorted, order): four of 8 or three of
+// 10 bits for 30-bit keys, eight for 63-bit ones
 void launch_sort(const StepBufs& b, cudaStream_t st);
-// the four passes on explicit buffers: keys_in -> (keys_out, vals_out), values start as
-// the identity; keys_tmp/vals_tmp hold passes 0 and 2
+// the 8-bit passes on explicit buffers: keys_in -> (keys_out, vals_out), values start as the
+// identity; the passes in between alternate with keys_tmp / vals_tmp
 // key_bits: the keys' width, which sets the number of passes; an odd number needs a third
 // key buffer keys_tmp2 (keys_in itself may serve: only the first pass reads it).
 void launch_sort_passes(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_out, uint32_t* keys_tmp,
@@ -129,12 +130,12 @@ void launch_sort_passes(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* v
                         int key_bits = 32, uint32_t* keys_tmp2 = nullptr);
 // per-system digit histograms of b.codes (when codes come from the host)
 void launch_code_hist(const StepBufs& b, cudaStream_t st);
-// gx_build.cu: gather leaves + bottom-up Karras build and aggregation
-// Morton codes and sort of one system of at most small_sort_max() particles in one
+// gx_step.cu: Morton codes and sort of one system of at most small_sort_max() particles in one
 // launch (8-bit digits); small_sort_prepare once per device.
 uint32_t small_sort_max();
 void small_sort_prepare();
 void launch_small_sort(const StepBufs& b, cudaStream_t st);
+// gx_build.cu: gather leaves + bottom-up Karras build and aggregation
 void launch_build(const StepBufs& b, int quad, cudaStream_t st);
 // Per-device set-up of the build kernels (their dynamic shared-memory limit); call with the
 // device current, before any stream capture.

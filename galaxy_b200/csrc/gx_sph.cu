@@ -837,8 +837,8 @@ __global__ void __launch_bounds__(kSphThreads, 6) k_sph_hydro(HydroArgs a) {
   // exact test r >= 2 max(h_i, h_j) is made again in the flush).
   // The reference's gather is 2 h_max wide, h_max of all gas; here the box is 2 h of the
   // largest h around, and a cell farther from the target than the reach of the target and
-  // of the cell's own largest h holds no neighbour and is passed over (its bounds padded by far more than the rounding of floor(x / cell); cells
-  // at the coordinates' limits are kept). 65,536 gas particles in a cube, where h at the
+  // of the cell's own largest h holds no neighbour and is passed over (its bounds padded by far
+  // more than the rounding of floor(x / cell); cells at the coordinates' limits are kept). 65,536 gas particles in a cube, where h at the
   // corners is twice the inner h: 700 -> 375 us.
   const auto near = [&](uint32_t b, int ox, int oy, int oz, double cell) {
     const double lim = 2.0 * fmax(h_i, static_cast<double>(__uint_as_float(a.hcell[b])));

@@ -6,23 +6,22 @@
 // its AABB and theta*(d - delta) >= s, s = 2*max(half extents); otherwise it is
 // opened) and :673-675 (result times G).
 //
-// One warp walks the tree for 32 Morton-consecutive targets of one system. The warp
-// visits the union of the 32 per-target walks (an explicit stack of (node, lane mask)
-// pairs kept in registers, entry j in lane j % 32); every node record is loaded once
-// per warp (a broadcast load) and each lane applies its OWN opening decision, so
-// every lane takes exactly the reference's set of terms for its target. A tree over
-// 30-bit (63-bit) codes with a 32-bit position tie-break is at most 63 (96) levels
-// deep, so 96 stack entries always suffice (overflow raises the device error word).
-//
-// FP32 mode: node centres of mass and leaf positions are float-float (hi + lo), so
-// dx = (c_hi - x_hi) + (c_lo - x_lo) keeps ~48 bits of the f64 coordinates; the
-// opening test compares d^2 with rcrit^2 = (s/theta + delta)^2 and re-decides in
-// FP64 with the reference's exact expression whenever the FP32 value lies within a
-// relative 4e-6 band of the threshold (or touches the AABB within 2^-20), so every
-// opening decision equals the reference's. Terms are accumulated in FP32 with Kahan
-// compensation.
-// FP64 mode: the reference's arithmetic, operation for operation and in its
-// depth-first order, so accelerations are bit-identical to the reference's CPU walk.
+// FP32 walk (k_walk_f32): one warp walks the tree for 8, 16 or 32 Morton-consecutive targets
+// of one system. It pops up to 32 nodes at a time from a stack in shared memory, one a lane,
+// decides each node's two children for all its targets against the targets' box, and lists
+// what they take; the lists are evaluated a batch at a time. Decisions that the box leaves
+// open are made for every target. Node centres of mass and leaf positions are float-float
+// (hi + lo), ~48 bits of the f64 coordinates; the opening test compares d^2 with
+// rcrit^2 = (s/theta + delta)^2 and re-decides in FP64 with the reference's exact expression
+// whenever the FP32 value lies within a relative 4e-6 band of the threshold (or touches the
+// AABB within 2^-20), so every opening decision equals the reference's. Terms are
+// accumulated in FP32 with Kahan compensation; the sums leave FP32 compensated.
+// FP64 walk (k_walk_f64): every lane walks the tree for its own target, without a stack (a
+// record names the node that follows its subtree), with the reference's arithmetic,
+// operation for operation and in its depth-first order, so accelerations are
+// bit-identical to the reference's CPU walk.
+// Bounds: the FP32 stack cannot pass kWalkStack, and the steps of either walk are limited by
+// the system's nodes; a tree that breaks them raises the device error word.
 #include "gx_kernels.h"
 
 namespace gx {
