@@ -35,7 +35,7 @@ constexpr size_t kSlot = size_t{1} << 20;
 constexpr int kSlots = 8;
 constexpr size_t kMinIn = size_t{1} << 19;
 constexpr size_t kOutCredit = size_t{1} << 17;
-constexpr size_t kCredit = size_t{32} << 20;
+constexpr size_t kCredit = size_t{16} << 20;
 constexpr size_t kPiece = size_t{1} << 17;  // bytes a thread moves at a time
 constexpr int kMaxBuffers = 4;
 

@@ -59,7 +59,7 @@ def test_pinned_arrays():
 @pytest.mark.parametrize("n", [1365, 1366, 2730, 2731, 21845, 21846])
 def test_sizes_around_the_rules(n):
     # Two outputs of 24 n bytes: to 64 KB together through the handle's buffer, otherwise
-    # staged; inputs of 24 n bytes from 512 KB on. A thread's first 32 MB go directly.
+    # staged; inputs of 24 n bytes from 512 KB on. A thread's first 16 MB go directly.
     _round_trip(400000, 1)
     _round_trip(n, n)
 
