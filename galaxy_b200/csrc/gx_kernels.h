@@ -70,14 +70,16 @@ struct StepBufs {
 constexpr int kWalkCtas = 4, kWalkCtasQuad = 4;
 
 // Launches kern after the kernel before it on st, to be scheduled as that one drains; kern
-// begins with step_kernel_begin. That takes about 1 us off the gap to the kernel before
-// it. Above kEarlyTiles tiles it is an ordinary launch: blocks placed while the kernel before
-// still runs land unevenly, which costs more than the gap (and more yet in the tree walk,
-// whose blocks run longest: up to 4%, so it never is launched early). A step of a disk, us,
-// ordinary / early: 2 tiles 222.8 / 214.7, 4 246.2 / 239.5, 8 311.6 / 309.1, 12 368.5 / 366.6,
-// 14 388.1 / 385.7, 16 427.2 / 432.1, 24 464.9 / 467.4, 48 700.9 / 710.6, 64 863 / 878, 80 1037 /
-// 1064; 16 systems of a tile 342.7 / 352.5, 40 of two 1010 / 1037.
-constexpr uint32_t kEarlyTiles = 12;
+// begins with step_kernel_begin. That hides the launch and the gap to the kernel before it. But
+// blocks placed while the kernel before still runs land unevenly, and the tree walk that ends
+// the step pays for it (more yet when it is launched early itself: up to 4%, so it never is).
+// Launched one by one, up to kEarlyTiles tiles gain: a step of a disk, us, ordinary / early: 16
+// tiles 465 / 446, 32 588 / 566, 48 754 / 742, 80 1093 / 1094; a force call's device time 16 tiles
+// 405 / 392, 48 703 / 697, 80 1076 / 1064; 96 tiles 1270 / 1280. In a replayed graph, whose
+// launches are cheap, only few do: 2 tiles 222.8 / 214.7, 4 246.2 / 239.5, 8 311.6 / 309.1, 12 368.5
+// / 366.6, 14 388.1 / 385.7, 16 427.2 / 432.1, 48 700.9 / 710.6, 80 1037 / 1064; 16 systems of a tile
+// 342.7 / 352.5, 40 of two 1010 / 1037.
+constexpr uint32_t kEarlyTiles = 80, kEarlyTilesGraph = 12;
 template <class... P, class... A>
 void launch_after(uint32_t ntiles, void (*kern)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute attr;
@@ -89,7 +91,9 @@ void launch_after(uint32_t ntiles, void (*kern)(P...), uint32_t grid, uint32_t b
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = ntiles <= kEarlyTiles ? 1 : 0;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (ntiles <= kEarlyTiles && ntiles > kEarlyTilesGraph) (void)cudaStreamIsCapturing(st, &cap);
+  cfg.numAttrs = ntiles <= (cap == cudaStreamCaptureStatusNone ? kEarlyTiles : kEarlyTilesGraph) ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
