@@ -134,8 +134,8 @@ int gx_accelerations_active(gx_handle* h, size_t n, const double* pos, const dou
  * positions: targets and leaf sources take pos / mass given here, internal nodes keep the
  * cached aggregates (the reference's "only far cell COMs are stale"). With unchanged
  * positions the result equals gx_accelerations_active. Any other force call or step on
- * the handle replaces the cached tree (GX_ERR_STATE until the next rebuild); n must equal
- * the cached n. */
+ * the handle replaces the cached tree, and a call for another number of particles or a stage
+ * call ends it (GX_ERR_STATE until the next rebuild); n must equal the cached n. */
 int gx_rebuild_gravity_cache(gx_handle* h, size_t n, const double* pos, const double* mass);
 int gx_gravity_active_cached(gx_handle* h, size_t n, const double* pos, const double* mass, size_t n_active,
                              const uint32_t* active, double* acc_out);
