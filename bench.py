@@ -677,10 +677,10 @@ def run_precision(args):
         dist.destroy_process_group()
 
 
-# Kernels a gas-mode step adds to the 9 of the gravity step when bucket numbers take four sort
-# passes: gather, scalars, 3 grids (keys, histogram, 4 sort passes, fill, mixed flags), seeds,
-# density cell, density, h_max, hydro cell, pack, hydro, scatter. Up to 2^24 buckets three
-# passes sort them (3 fewer), and the reach kernel adds one.
+# Kernels a gas-mode step adds to the 9 of the gravity step. First count: gather, scalars, 3
+# grids (keys, histogram, 4 sort passes, fill, mixed flags), seeds, density cell, density,
+# h_max, hydro cell, pack, hydro, scatter. Now up to 2^24 buckets three passes sort a grid (3
+# fewer) and the reach kernel adds one.
 SPH_LAUNCHES_PER_STEP = 2 + 3 * 8 + 8
 SPH_LAUNCHES_NOW = SPH_LAUNCHES_PER_STEP - 3 + 1
 
